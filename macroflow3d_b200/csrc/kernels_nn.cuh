@@ -61,7 +61,31 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
                  "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
                  : "memory");
 }
+// One lane of the warp, the same one for the same (full) mask.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r;
+}
+// The same product, called by a whole warp in uniform control flow and issued by its elected lane:
+// the descriptors then stay in uniform registers.  From one lane's own branch every product
+// moved its descriptors there first, which took longer than the product (16 -> 16 channels at 128^3:
+// 127 cycles a product).  Descriptors as (low, high) words; only the low one carries the start address.
+__device__ __forceinline__ void umma_bf16_warp(uint32_t d_tmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
+                                               uint32_t idesc, uint32_t accumulate, uint32_t leader) {
+    asm volatile("{\n .reg .pred p, q;\n .reg .b64 da, db;\n setp.ne.b32 p, %6, 0;\n setp.ne.b32 q, %7, 0;\n"
+                 " mov.b64 da, {%1, %2};\n mov.b64 db, {%3, %4};\n"
+                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(d_tmem),
+                 "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate), "r"(leader)
+                 : "memory");
+}
 // arrive on an mbarrier once every tcgen05.mma this thread issued before has completed
+__device__ __forceinline__ void umma_commit_warp(uint64_t* bar, uint32_t leader) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+                 " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(sm_u32(bar)),
+                 "r"(leader)
+                 : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sm_u32(bar))
                  : "memory");
@@ -331,7 +355,7 @@ struct BrickArgs {
 template <int A>
 __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a, const BrickArgs g) {
     extern __shared__ __align__(1024) unsigned char br_sm[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int cin = a.cin, ctot = a.cout, nhg = cin / 8;
     const int NP = g.NP, co0 = g.co0, coutp = g.coutp, zchunk = g.zchunk;
     const int W = 8 * A + 2;                       // slot width in voxels
@@ -355,9 +379,10 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
     // 16 B, 8-row groups 128 B apart, one region of coutp rows per 8 input channels
     for (int q = tid; q < 27 * coutp * nhg; q += BR_NT) {
         const int t = q / (coutp * nhg), r = q % (coutp * nhg), n = r / nhg, hg = r % nhg;
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.w + ((size_t)(co0 + n) * 27 + t) * cin) + hg);
-        *reinterpret_cast<uint4*>(wsm + ((size_t)(t * nhg + hg) * coutp + n) * 16) = v;
+        cp_async16(sm_u32(wsm) + (uint32_t)(((t * nhg + hg) * coutp + n) * 16),
+                   a.w + ((size_t)(co0 + n) * 27 + t) * cin + hg * 8, true);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (warp == mma_warp) {
         tmem_alloc(tmem_slot, ncols);
         tmem_relinquish();
@@ -394,7 +419,7 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
         unsigned pc = 0;          // planes staged so far (ring position)
         const int K = NP - 3;     // planes whose copies stay in flight (3 slots are being read)
         int pend[BR_MAXNP] = {}, np_ = 0, ph = 0; // committed, not yet announced slots (oldest at ph)
-        const int nchunk = nhg * W * 18;
+        const uint32_t inv_h = (65536u + nhg - 1) / nhg; // q / nhg by a multiply, exact for q < 4096
         // wait until at most n copy groups of this thread are pending
         auto wait_groups = [](int n) {
             switch (n) {
@@ -430,12 +455,18 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
                 }
                 const uint32_t base = sm_u32(slots + (size_t)sl * SLOT);
                 const bool pin = p >= 0 && p < nz;
-                for (int q = tid; q < nchunk; q += BR_PROD * 32) {
-                    const int hg = q / (W * 18), r = q % (W * 18), yy = r / W, xx = r % W;
-                    const int gx = x0 - 1 + xx, gy = y0 - 1 + yy;
-                    const bool ok = pin && gx >= 0 && gx < nx && gy >= 0 && gy < ny;
-                    const __nv_bfloat16* src = ok ? a.x + (((size_t)p * ny + gy) * nx + gx) * cin + hg * 8 : a.x;
-                    cp_async16(base + (uint32_t)(hg * REG + r * 16), src, ok);
+                // a warp takes a row of voxels at a time, lanes along (voxel, 8 channels): a row
+                // is read as consecutive 16-byte pieces
+                for (int yy = warp; yy < 18; yy += BR_PROD) {
+                    const int gy = y0 - 1 + yy;
+                    const bool rin = pin && gy >= 0 && gy < ny;
+                    const __nv_bfloat16* row = a.x + ((long long)(rin ? p : 0) * ny + (rin ? gy : 0)) * nx * cin;
+                    const uint32_t dst = base + (uint32_t)(yy * W * 16);
+                    for (int q = lane; q < W * nhg; q += 32) {
+                        const int xx = (int)((q * inv_h) >> 16), hg = q - xx * nhg, gx = x0 - 1 + xx;
+                        const bool ok = rin && gx >= 0 && gx < nx;
+                        cp_async16(dst + (uint32_t)(hg * REG + xx * 16), ok ? row + (long long)gx * cin + hg * 8 : a.x, ok);
+                    }
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
                 pend[(ph + np_) % BR_MAXNP] = sl;
@@ -446,64 +477,68 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
         while (np_ > 0) publish_oldest(); // the last planes
         if (fail) atomicExch(s_fail, 1);
     } else if (warp == mma_warp) {
-        // ---------------- MMA issuer (one thread) ----------------
-        if (lane == 0) {
-            const uint32_t idesc = idesc_bf16(CONV_TM, coutp);
-            const uint64_t bbase = kdesc(sm_u32(wsm), (uint32_t)(coutp * 16), 128u);
-            unsigned pc = 0, pw = 0; // planes waited for, output planes done
-            for (int br = blockIdx.x; br < nbricks && !fail; br += gridDim.x) {
-                const int zc = br / (bx * by);
-                const int z0 = zc * zchunk, z1 = min(nz, z0 + zchunk);
-                const unsigned pfirst = pc; // ring position of plane z0 - 1
-                for (int k = 0; k < 2 && !fail; ++k, ++pc)
-                    if (!nn_mbar_wait(&full[pc % NP], (pc / NP) & 1u)) fail = true;
-                for (int z = z0; z < z1 && !fail; ++z, ++pw) {
-                    if (!nn_mbar_wait(&full[pc % NP], (pc / NP) & 1u)) { // plane z + 1
-                        fail = true;
-                        break;
-                    }
-                    ++pc;
-                    const int tb = (int)(pw & 1u);
-                    if (pw >= 2 && !nn_mbar_wait(&tempty[tb], ((pw / 2) - 1) & 1u)) {
-                        fail = true;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t dacc = tmem + (uint32_t)(tb * A * coutp);
-                    // descriptors differ only in their start address (bits 0-13, in 16-byte
-                    // units): one base per operand, offsets added
-                    for (int dz = -1; dz <= 1; ++dz) {
-                        const unsigned pr = pfirst + (unsigned)(z - z0 + 1 + dz); // ring position of plane z + dz
-                        const uint64_t abase = kdesc(sm_u32(slots + (size_t)(pr % NP) * SLOT), (uint32_t)REG,
-                                                     (uint32_t)(W * 16));
-                        const int tz = (dz + 1) * 9;
-                        for (int s2 = 0; s2 < cin / 16; ++s2) {
-                            const uint64_t a_s = abase + (uint64_t)(2 * s2 * (REG >> 4));
-                            const uint64_t b_s = bbase + (uint64_t)(2 * s2 * coutp);
+        // ---------------- MMA issuer (one warp, its elected lane issues) ----------------
+        const uint32_t leader = elect_one();
+        const uint32_t idesc = idesc_bf16(CONV_TM, coutp);
+        const uint64_t bbase = kdesc(sm_u32(wsm), (uint32_t)(coutp * 16), 128u);
+        const uint32_t bhi = (uint32_t)(bbase >> 32), tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+        unsigned pc = 0, pw = 0; // planes waited for, output planes done
+        for (int br = blockIdx.x; br < nbricks && !fail; br += gridDim.x) {
+            const int zc = br / (bx * by);
+            const int z0 = zc * zchunk, z1 = min(nz, z0 + zchunk);
+            const unsigned pfirst = pc; // ring position of plane z0 - 1
+            auto wait_full = [&](unsigned p) {
+                return __all_sync(0xffffffffu, nn_mbar_wait(&full[p % NP], (p / NP) & 1u)) != 0;
+            };
+            for (int k = 0; k < 2 && !fail; ++k, ++pc)
+                if (!wait_full(pc)) fail = true;
+            for (int z = z0; z < z1 && !fail; ++z, ++pw) {
+                if (!wait_full(pc)) { // plane z + 1
+                    fail = true;
+                    break;
+                }
+                ++pc;
+                const int tb = (int)(pw & 1u);
+                if (pw >= 2 && !__all_sync(0xffffffffu, nn_mbar_wait(&tempty[tb], ((pw / 2) - 1) & 1u))) {
+                    fail = true;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t dacc = tmem_u + (uint32_t)(tb * A * coutp);
+                // descriptors differ only in their start address (bits 0-13, in 16-byte
+                // units): one base per operand, offsets added
+                for (int dz = -1; dz <= 1; ++dz) {
+                    const unsigned pr = pfirst + (unsigned)(z - z0 + 1 + dz); // ring position of plane z + dz
+                    const uint64_t abase = kdesc(sm_u32(slots + (size_t)(pr % NP) * SLOT), (uint32_t)REG,
+                                                 (uint32_t)(W * 16));
+                    const uint32_t ahi = (uint32_t)(abase >> 32);
+                    const int tz = (dz + 1) * 9;
+                    for (int s2 = 0; s2 < cin / 16; ++s2) {
+                        const uint32_t a_s = (uint32_t)abase + (uint32_t)(2 * s2 * (REG >> 4));
+                        const uint32_t b_s = (uint32_t)bbase + (uint32_t)(2 * s2 * coutp + tz * nhg * coutp);
 #pragma unroll
-                            for (int tyx = 0; tyx < 9; ++tyx) {
-                                const int dy = tyx / 3, dx = tyx % 3; // 0..2: offsets + 1
-                                const uint64_t bd = b_s + (uint64_t)((tz + tyx) * nhg * coutp);
-                                // every tile's first product of the plane overwrites its accumulator
-                                const uint32_t acc = (dz > -1 || s2 > 0 || tyx > 0) ? 1u : 0u;
+                        for (int tyx = 0; tyx < 9; ++tyx) {
+                            const int dy = tyx / 3, dx = tyx % 3; // 0..2: offsets + 1
+                            const uint32_t bd = b_s + (uint32_t)(tyx * nhg * coutp);
+                            // every tile's first product of the plane overwrites its accumulator
+                            const uint32_t acc = (dz > -1 || s2 > 0 || tyx > 0) ? 1u : 0u;
 #pragma unroll
-                                for (int j = 0; j < A; ++j)
-                                    umma_bf16(dacc + (uint32_t)(j * coutp), a_s + (uint64_t)(dy * W + dx + 8 * j), bd,
-                                              idesc, acc);
-                            }
+                            for (int j = 0; j < A; ++j)
+                                umma_bf16_warp(dacc + (uint32_t)(j * coutp), a_s + (uint32_t)(dy * W + dx + 8 * j), ahi,
+                                               bd, bhi, idesc, acc, leader);
                         }
                     }
-                    umma_commit(&tfull[tb]);
-                    // plane z - 1 is read by no later output plane of this brick
-                    umma_commit(&empty[(pfirst + (unsigned)(z - z0)) % NP]);
                 }
-                if (!fail) { // the brick's last two planes (z1 - 1, z1) are released too
-                    umma_commit(&empty[(pfirst + (unsigned)(z1 - z0)) % NP]);
-                    umma_commit(&empty[(pfirst + (unsigned)(z1 - z0 + 1)) % NP]);
-                }
+                umma_commit_warp(&tfull[tb], leader);
+                // plane z - 1 is read by no later output plane of this brick
+                umma_commit_warp(&empty[(pfirst + (unsigned)(z - z0)) % NP], leader);
             }
-            if (fail) atomicExch(s_fail, 1);
+            if (!fail) { // the brick's last two planes (z1 - 1, z1) are released too
+                umma_commit_warp(&empty[(pfirst + (unsigned)(z1 - z0)) % NP], leader);
+                umma_commit_warp(&empty[(pfirst + (unsigned)(z1 - z0 + 1)) % NP], leader);
+            }
         }
+        if (fail && lane == 0) atomicExch(s_fail, 1);
     } else {
         // ---------------- epilogue warps: TMEM -> registers -> global ----------------
         const int q = warp & 3;      // TMEM lane quarter this warp may access
@@ -573,8 +608,8 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
     // ---- teardown: every role has stopped issuing; the MMAs still in flight are waited for
     // (one more commit tracks all of them) before the accumulator is released ----
     __syncthreads();
-    if (warp == mma_warp && lane == 0) {
-        umma_commit(drain);
+    if (warp == mma_warp) { // (the lane that issued them commits)
+        umma_commit_warp(drain, elect_one());
         if (!nn_mbar_wait(drain, 0u)) atomicExch(s_fail, 1);
     }
     __syncthreads();
@@ -587,128 +622,282 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
     }
 }
 
-// ---- weight gradient (CUDA cores, FP32): dW[co][t][ci] = sum_v dY[v][co] X[v + off(t)][ci] ----
-// One CTA per (tap, voxel chunk); the CTA's partial goes to part[chunk][co][t][ci] and
-// wgrad_reduce_kernel adds the chunks in order (deterministic).  Each thread owns 4 x 4
-// (co, ci) outputs; when the layer has fewer than 256 such tiles, G thread groups split the
-// staged voxels and their sums are added in shared memory at the end.
-constexpr int WG_NT = 256;
-constexpr int WG_VOX = 32; // voxels staged per step
-__global__ void __launch_bounds__(WG_NT) wgrad_kernel(const __nv_bfloat16* __restrict__ x,
-                                                      const __nv_bfloat16* __restrict__ dy, float* __restrict__ part,
-                                                      int nx, int ny, int nz, int cin, int cout, int vox_per_chunk) {
-    __shared__ __align__(16) float sx[WG_VOX][CONV_MAXC];
-    __shared__ __align__(16) float sd[WG_VOX][CONV_MAXC];
-    __shared__ __align__(16) float red[WG_NT * 16];
-    const int t = blockIdx.x, chunk = blockIdx.y;
-    const int dz = t / 9 - 1, dyo = (t / 3) % 3 - 1, dxo = t % 3 - 1;
-    const long long V = (long long)nx * ny * nz;
-    const long long v0 = (long long)chunk * vox_per_chunk, v1 = min(V, v0 + vox_per_chunk);
-    const int tci = cin / 4, ntile = (cout / 4) * tci;
-    const int G = ntile >= WG_NT ? 1 : WG_NT / ntile; // thread groups over the voxels
-    const int per = (ntile + WG_NT - 1) / WG_NT;      // tiles per thread (G == 1)
-    const int tid = threadIdx.x, grp = tid / (WG_NT / G), tin = tid % (WG_NT / G);
-    const bool active = tid < G * (WG_NT / G) && (G > 1 ? tin < ntile : true);
-    float acc[2][16];
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int i = 0; i < 16; ++i) acc[u][i] = 0.f;
-    for (long long vb = v0; vb < v1; vb += WG_VOX) {
-        __syncthreads();
-        for (int e = tid; e < WG_VOX * (cin / 8); e += WG_NT) {
-            const int q = e / (cin / 8), c8 = e % (cin / 8);
-            const long long v = vb + q;
-            uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-            if (v < v1) {
-                const int i = (int)(v % nx) + dxo, j = (int)((v / nx) % ny) + dyo, k = (int)(v / ((long long)nx * ny)) + dz;
-                if (i >= 0 && i < nx && j >= 0 && j < ny && k >= 0 && k < nz)
-                    raw = __ldg(reinterpret_cast<const uint4*>(x + ((size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k)) * cin) + c8);
-            }
-            const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) sx[q][c8 * 8 + u] = __bfloat162float(b[u]);
-        }
-        for (int e = tid; e < WG_VOX * (cout / 8); e += WG_NT) {
-            const int q = e / (cout / 8), c8 = e % (cout / 8);
-            const long long v = vb + q;
-            uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-            if (v < v1) raw = __ldg(reinterpret_cast<const uint4*>(dy + (size_t)v * cout) + c8);
-            const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) sd[q][c8 * 8 + u] = __bfloat162float(b[u]);
-        }
-        __syncthreads();
-        if (!active) continue;
-        for (int u = 0; u < per && u < 2; ++u) {
-            const int tile = G > 1 ? tin : tid + u * WG_NT;
-            if (tile >= ntile) break;
-            const int co0 = (tile / tci) * 4, ci0 = (tile % tci) * 4;
-            for (int q = grp; q < WG_VOX; q += G) {
-                const float4 d4 = *reinterpret_cast<const float4*>(&sd[q][co0]);
-                const float4 x4 = *reinterpret_cast<const float4*>(&sx[q][ci0]);
-                const float dv[4] = {d4.x, d4.y, d4.z, d4.w}, xv[4] = {x4.x, x4.y, x4.z, x4.w};
-#pragma unroll
-                for (int a2 = 0; a2 < 4; ++a2)
-#pragma unroll
-                    for (int b2 = 0; b2 < 4; ++b2) acc[u][a2 * 4 + b2] += dv[a2] * xv[b2];
-            }
-        }
-    }
-    // sum the G groups (index order), then store the tile
-    if (G > 1) {
-        __syncthreads();
-        if (active)
-#pragma unroll
-            for (int i = 0; i < 16; ++i) red[tid * 16 + i] = acc[0][i];
-        __syncthreads();
-        if (active && grp == 0) {
-            for (int g2 = 1; g2 < G; ++g2)
-#pragma unroll
-                for (int i = 0; i < 16; ++i) acc[0][i] += red[(g2 * (WG_NT / G) + tin) * 16 + i];
-        }
-    }
-    if (!active || (G > 1 && grp != 0)) return;
-    for (int u = 0; u < per && u < 2; ++u) {
-        const int tile = G > 1 ? tin : tid + u * WG_NT;
-        if (tile >= ntile) break;
-        const int co0 = (tile / tci) * 4, ci0 = (tile % tci) * 4;
-#pragma unroll
-        for (int a2 = 0; a2 < 4; ++a2)
-#pragma unroll
-            for (int b2 = 0; b2 < 4; ++b2)
-                part[((size_t)chunk * cout + co0 + a2) * 27 * cin + (size_t)t * cin + ci0 + b2] = acc[u][a2 * 4 + b2];
-    }
+// ---- weight gradient: dW[co][t][ci] = sum_v dY[v][co] X[v + off(t)][ci] ----
+// A contraction over the voxels (K), so both operands are read channel-major ("MN-major") and
+// the activations need no transposition: in a staged plane, one region per 8 channels with a
+// voxel's 16 bytes at consecutive addresses, 8 consecutive voxels are one core matrix.
+//   M = 128 rows: 16 consecutive 8-channel regions of X, which run over the channels of a plane
+//     and then over the next planes; the dz taps of a voxel plane are 3 planes, so one product
+//     covers all three (and, with Q voxel planes in N, all Q + 2).  Rows past them are unused.
+//   N = Q * coN columns: the output channels of Q consecutive voxel planes of dY.
+//   K = 16 voxels along x; the dy and dx taps are shifted start addresses of X.
+// The Q voxel planes' blocks of the result are separate partial sums (row plane p and column
+// plane q belong to tap dz = p - q).  A CTA walks voxel bricks (16 x BY x BZ, two in flight where
+// shared memory allows) with an accumulator per (dy, dx) and M tile in TMEM.  The tensor core truncates
+// when it adds to an accumulator, and a chain of n products loses about 1.3e-8 n of its sum (measured:
+// 304 products 4.0e-6, 913 products 1.4e-5), so after every BY products the accumulators are added to
+// 32-bit sums in registers (rounded to nearest) and start again at zero: 8e-8 over 128^3 voxels,
+// against 1.1e-7 for chains of 32-bit multiply-adds.
+// Each CTA's sums go to part[chunk * Q + q] and wgrad_reduce_kernel adds those in a fixed order.  The bias
+// gradient is summed from the staged dY on the CUDA cores while the tensor core runs.
+// Bound by the products (an A tile of 4 KB each, 90 to 140 cycles at 16 to 32 columns).  The twelve layers of
+// a 128^3 sample: 2.1 ms, against 29.6 ms as FP32 register tiles on the CUDA cores (and 1.3 ms for
+// their bias gradients, which are now part of it); 16 -> 16 channels at 128^3: 0.29 ms.
+constexpr int WG_NT = 512;
+constexpr int WG_COLS = 320; // accumulator columns, at most: 5 groups of 16 per warp, 80 registers
+constexpr int WG_BX = 16, WG_XW = WG_BX + 2;
+struct WgArgs {
+    const __nv_bfloat16* x;  // [V][cin]
+    const __nv_bfloat16* dy; // [V][cout]
+    float* part;             // [nchunks * Q][cout][27][cin]
+    float* bpart;            // [nchunks][cout]
+    int nx, ny, nz, cin, cout;
+    int Q, tiles, coN; // voxel planes in N, M tiles, output channels per CTA
+    int BY, BZ, stages;     // brick rows and planes (BZ a multiple of Q), bricks staged at a time
+    int* err;               // set when an mbarrier wait gives up
+};
+__host__ __device__ constexpr int wg_xreg(int BY) { return WG_XW * (BY + 2) * 16; } // one 8-channel region of a plane
+__host__ __device__ constexpr int wg_yreg(int BY) { return WG_BX * BY * 16; }
+__host__ __device__ constexpr size_t wg_xbytes(int cin, int BY, int BZ) {
+    return (size_t)(BZ + 2) * (cin / 8) * wg_xreg(BY);
+}
+__host__ __device__ constexpr size_t wg_ybytes(int coN, int BY, int BZ) {
+    return (size_t)BZ * (coN / 8) * wg_yreg(BY);
+}
+// shared memory of a launch: the bricks, and what the unused rows of the last one read past it
+constexpr size_t wg_smem(int cin, int coN, int Q, int tiles, int BY, int BZ, int stages) {
+    const long long xb = (long long)wg_xbytes(cin, BY, BZ), yb = (long long)wg_ybytes(coN, BY, BZ);
+    const long long over = (16ll * tiles - (long long)(Q + 2) * (cin / 8)) * wg_xreg(BY);
+    return (size_t)((stages - 1) * (xb + yb) + xb + (over > yb ? over : yb));
 }
 
-// dw (+)= sum over chunks of the partials, in chunk order (deterministic); used for the
-// weight and the bias partials
-__global__ void wgrad_reduce_kernel(const float* __restrict__ part, int nchunks, size_t n, float* __restrict__ dw,
-                                    int accumulate) {
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int c = 0; c < nchunks; ++c) s += part[(size_t)c * n + e];
-        dw[e] = accumulate ? dw[e] + s : s;
+template <int NDT>
+__global__ void __launch_bounds__(WG_NT, 1) wgrad_tc_kernel(const WgArgs a) {
+    extern __shared__ __align__(1024) unsigned char wg_sm[];
+    __shared__ __align__(8) uint64_t bar; // the products issued last have completed
+    __shared__ uint32_t tmem_slot;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int cin = a.cin, cout = a.cout, nhg = cin / 8, coN = a.coN, nho = coN / 8, Q = a.Q, tiles = a.tiles;
+    const int BY = a.BY, BZ = a.BZ, stages = a.stages;
+    constexpr int ndt = NDT; // 9: every (dy, dx); 3: dy = blockIdx.y, every dx
+    const int co0 = blockIdx.z * coN, td0 = blockIdx.y * ndt;
+    const int nx = a.nx, ny = a.ny, nz = a.nz;
+    const int XREG = wg_xreg(BY), YREG = wg_yreg(BY);
+    const uint32_t xbytes = (uint32_t)wg_xbytes(cin, BY, BZ), sbytes = xbytes + (uint32_t)wg_ybytes(coN, BY, BZ);
+    const uint32_t base = sm_u32(wg_sm);
+    const int ncol = Q * coN;
+    const uint32_t ncols = tmem_cols(ndt * tiles * ncol);
+    if (warp == 0) {
+        tmem_alloc(&tmem_slot, ncols);
+        tmem_relinquish();
     }
-}
+    if (tid == 0) {
+        nn_mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot, tmem_u = __shfl_sync(0xffffffffu, tmem, 0), leader = elect_one();
+    const int nbx = (nx + WG_BX - 1) / WG_BX, nby = (ny + BY - 1) / BY, nbz = (nz + BZ - 1) / BZ;
+    const int nblk = nbx * nby * nbz;
 
-// bias gradient partials: part[chunk][co] = sum over the chunk's voxels of dY[v][co]
-__global__ void bgrad_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ part, long long V, int cout,
-                             int vox_per_chunk) {
-    __shared__ float red[256];
-    const int chunk = blockIdx.x;
-    const long long v0 = (long long)chunk * vox_per_chunk, v1 = min(V, v0 + vox_per_chunk);
-    for (int co = 0; co < cout; ++co) {
-        float s = 0.f;
-        for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) s += __bfloat162float(dy[(size_t)v * cout + co]);
-        red[threadIdx.x] = s;
+    // copies of one brick: a warp takes a row of voxels at a time, lanes along (voxel, 8 channels),
+    // so that a row is read as consecutive 16-byte pieces; zeros outside the grid
+    const uint32_t inv_h = (65536u + nhg - 1) / nhg, inv_o = (65536u + nho - 1) / nho; // exact for < 4096
+    auto load = [&](int b, int buf) {
+        const int x0 = (b % nbx) * WG_BX, y0 = ((b / nbx) % nby) * BY, z0 = (b / (nbx * nby)) * BZ;
+        const uint32_t xs = base + buf * sbytes, ys = xs + xbytes;
+        const int xrows = (BZ + 2) * (BY + 2), xlen = WG_XW * nhg;
+        for (int r = warp; r < xrows; r += WG_NT / 32) {
+            const int pz = r / (BY + 2), yy = r - pz * (BY + 2);
+            const int gz = z0 + pz - 1, gy = y0 + yy - 1;
+            const bool rin = gz >= 0 && gz < nz && gy >= 0 && gy < ny;
+            const __nv_bfloat16* row = a.x + ((long long)(rin ? gz : 0) * ny + (rin ? gy : 0)) * nx * cin;
+            const uint32_t dst = xs + (uint32_t)(pz * nhg * XREG + yy * (WG_XW * 16));
+            for (int q = lane; q < xlen; q += 32) {
+                const int xx = (int)((q * inv_h) >> 16), hg = q - xx * nhg, gx = x0 + xx - 1;
+                const bool ok = rin && gx >= 0 && gx < nx;
+                cp_async16(dst + (uint32_t)(hg * XREG + xx * 16), ok ? row + (long long)gx * cin + hg * 8 : a.x, ok);
+            }
+        }
+        const int yrows = BZ * BY, ylen = WG_BX * nho;
+        for (int r = warp; r < yrows; r += WG_NT / 32) {
+            const int pz = r / BY, yy = r - pz * BY;
+            const int gz = z0 + pz, gy = y0 + yy;
+            const bool rin = gz < nz && gy < ny;
+            const __nv_bfloat16* row = a.dy + ((long long)(rin ? gz : 0) * ny + (rin ? gy : 0)) * nx * cout + co0;
+            const uint32_t dst = ys + (uint32_t)(pz * nho * YREG + yy * (WG_BX * 16));
+            for (int q = lane; q < ylen; q += 32) {
+                const int xx = (int)((q * inv_o) >> 16), hg = q - xx * nho, gx = x0 + xx;
+                const bool ok = rin && gx < nx;
+                cp_async16(dst + (uint32_t)(hg * YREG + xx * 16), ok ? row + (long long)gx * cout + hg * 8 : a.dy, ok);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // bias gradient: a thread sums one 8-channel group over a strided share of the brick's voxels
+    const bool bias = blockIdx.y == 0;
+    int per = WG_NT / 2; // threads per group, a power of two
+    while (per * nho > WG_NT) per >>= 1;
+    const int bhg = tid / per, bsub = tid % per;
+    float bacc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) bacc[i] = 0.f;
+
+    const uint32_t idesc = idesc_bf16(CONV_TM, ncol) | (1u << 15) | (1u << 16); // A and B MN-major
+    // this warp's accumulator columns: groups of 16, every 4th (four warps share a lane quarter)
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const int groups = ndt * tiles * (ncol / 16);
+    constexpr int GW = WG_COLS / 64;
+    float sum[GW][16];
+#pragma unroll
+    for (int e = 0; e < GW; ++e)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum[e][i] = 0.f;
+    unsigned phase = 0u;
+    bool fail = false;
+    if ((int)blockIdx.x < nblk) load(blockIdx.x, 0);
+    int buf = 0;
+    for (int b = blockIdx.x; b < nblk && !fail; b += gridDim.x) {
+        const int bn = b + gridDim.x;
+        const bool ahead = stages == 2 && bn < nblk;
+        if (ahead) { // (the other buffer was left before the last barrier)
+            load(bn, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+        const uint32_t xs = base + buf * sbytes, ys = xs + xbytes;
+        const uint64_t ad0 = kdesc(xs, 128u, (uint32_t)XREG), bd0 = kdesc(ys, 128u, (uint32_t)YREG);
+        const uint32_t ahi = (uint32_t)(ad0 >> 32), bhi = (uint32_t)(bd0 >> 32);
+        const uint32_t a0 = (uint32_t)ad0 + (NDT == 9 ? 0u : (uint32_t)(blockIdx.y * WG_XW));
+        for (int zq = 0; zq < BZ; zq += Q) {
+            if (warp == 0) {
+                tc_fence_after();
+                for (int y = 0; y < BY; ++y) {
+                    const uint32_t bd = (uint32_t)bd0 + (uint32_t)((zq * nho * YREG + y * (WG_BX * 16)) >> 4);
+                    const uint32_t ay = a0 + (uint32_t)((zq * nhg * XREG) >> 4) + (uint32_t)(y * WG_XW);
+                    for (int tl = 0; tl < tiles; ++tl)
+#pragma unroll
+                        for (int d = 0; d < NDT; ++d) // (dy, dx) = (d / 3, d % 3), offsets + 1
+                            umma_bf16_warp(tmem_u + (uint32_t)((d * tiles + tl) * ncol),
+                                           ay + (uint32_t)(tl * XREG) + (uint32_t)((d / 3) * WG_XW + d % 3), ahi, bd, bhi,
+                                           idesc, y > 0 ? 1u : 0u, leader);
+                }
+                umma_commit_warp(&bar, leader);
+            }
+            if (bias && bhg < nho) { // the bias gradient's share of these planes, meanwhile
+                const unsigned char* yb = wg_sm + buf * sbytes + xbytes;
+                for (int z = zq; z < zq + Q; ++z) {
+                    const uint4* row = reinterpret_cast<const uint4*>(yb + (size_t)(z * nho + bhg) * YREG);
+                    for (int v = bsub; v < WG_BX * BY; v += per) {
+                        const uint4 raw = row[v];
+                        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&raw);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) bacc[i] += __bfloat162float(e[i]);
+                    }
+                }
+            }
+            __syncwarp();
+            if (!nn_mbar_wait(&bar, phase)) fail = true;
+            phase ^= 1u;
+            tc_fence_after();
+            if (!__any_sync(0xffffffffu, fail)) {
+#pragma unroll
+                for (int e = 0; e < GW; ++e) {
+                    const int g = (warp >> 2) + 4 * e;
+                    if (g < groups) { // (warp-uniform)
+                        float v[16];
+                        tmem_ld16(lane_base + (uint32_t)(g * 16), v);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) sum[e][i] += v[i];
+                    }
+                }
+            }
+            tc_fence_before();
+            // the accumulators are read (and, after the last planes, the buffer is left)
+            fail = __syncthreads_or(fail);
+            if (fail) break;
+        }
+        if (stages == 1 && bn < nblk && !fail) load(bn, 0);
+        if (stages == 2) buf ^= 1;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (!fail) {
+        const int m = (warp & 3) * 32 + lane;
+#pragma unroll
+        for (int e = 0; e < GW; ++e) {
+            const int gi = (warp >> 2) + 4 * e;
+            if (gi >= groups) break;
+            const int dt = gi / (ncol / 16), c0 = (gi % (ncol / 16)) * 16;
+            const int d = dt / tiles, tl = dt % tiles;
+            const int g = 16 * tl + (m >> 3), qq = c0 / coN, dz = g / nhg - qq;
+            if (dz >= 0 && dz <= 2) {
+                const int ci = (g % nhg) * 8 + (m & 7), t = dz * 9 + td0 + d, co = co0 + c0 - qq * coN;
+                float* o = a.part + (((size_t)blockIdx.x * Q + qq) * cout + co) * 27 * cin + (size_t)t * cin + ci;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) o[(size_t)i * 27 * cin] = sum[e][i];
+            }
+        }
+        if (bias) { // lanes of one channel group, then the warps, in index order
+            float(*bred)[CONV_MAXC] = reinterpret_cast<float(*)[CONV_MAXC]>(wg_sm); // (the bricks are done with)
+            for (int w = tid; w < (WG_NT / 32) * CONV_MAXC; w += WG_NT) bred[w / CONV_MAXC][w % CONV_MAXC] = 0.f;
             __syncthreads();
+            // a warp may hold the lanes of several channel groups (per < 32)
+            const int span = per < 32 ? per : 32;
+            for (int o = span >> 1; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float other = __shfl_down_sync(0xffffffffu, bacc[i], o);
+                    if ((lane & (span - 1)) + o < span) bacc[i] += other;
+                }
+            if (bhg < nho && (lane & (span - 1)) == 0)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) bred[warp][bhg * 8 + i] = bacc[i];
+            __syncthreads();
+            for (int c = tid; c < coN; c += WG_NT) {
+                float s = 0.f;
+                for (int w = 0; w < WG_NT / 32; ++w) s += bred[w][c];
+                a.bpart[(size_t)blockIdx.x * cout + co0 + c] = s;
+            }
         }
-        if (threadIdx.x == 0) part[(size_t)chunk * cout + co] = red[0];
-        __syncthreads();
+    } else if (tid == 0) {
+        atomicExch(a.err, 1);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, ncols);
+    }
+}
+
+// dw (+)= sum over np partials of n values, db (+)= sum over nb partials of m values: 32 values
+// per block, 8 threads a value, each over every 8th partial, then the 8 in order (deterministic)
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ part, int np, size_t n,
+                                                           float* __restrict__ dw, const float* __restrict__ bpart,
+                                                           int nb, int m, float* __restrict__ db, int accumulate) {
+    __shared__ float red[8][33];
+    const size_t nblk = (n + 31) / 32;
+    const bool w = blockIdx.x < nblk;
+    const size_t e = (w ? (size_t)blockIdx.x : (size_t)blockIdx.x - nblk) * 32 + threadIdx.x, len = w ? n : (size_t)m;
+    const float* src = w ? part : bpart;
+    float* dst = w ? dw : db;
+    const int cnt = w ? np : nb;
+    float s = 0.f;
+    if (e < len) {
+#pragma unroll 4
+        for (int c = threadIdx.y; c < cnt; c += 8) s += src[(size_t)c * len + e];
+    }
+    red[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0 && e < len) {
+#pragma unroll
+        for (int k = 1; k < 8; ++k) s += red[k][threadIdx.x];
+        dst[e] = accumulate ? dst[e] + s : s;
     }
 }
 

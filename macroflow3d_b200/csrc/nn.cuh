@@ -169,6 +169,20 @@ class WarmStartNet {
         return loss / count;
     }
 
+    // Planes per brick: the split of nz whose busiest CTA stages the fewest planes (its bricks' output
+    // planes and two halo planes each); at least 2 output planes a brick.
+    static int brick_zchunk(int cols, int nz, int sms) {
+        int best = nz;
+        long long cost = -1;
+        for (int nzc = 1; nzc <= std::max(1, nz / 2); ++nzc) {
+            const int zc = (nz + nzc - 1) / nzc;
+            const long long bricks = (long long)cols * ((nz + zc - 1) / zc);
+            const long long c = ((bricks + sms - 1) / sms) * (zc + 2);
+            if (cost < 0 || c < cost) cost = c, best = zc;
+        }
+        return best;
+    }
+
     // ---- single operations (tests) ----
     static void conv(cudaStream_t s, const Dims& d, int cin, int cout, const __nv_bfloat16* x,
                      const __nv_bfloat16* w, const float* bias, int relu, const __nv_bfloat16* mask, int y_f32,
@@ -208,12 +222,11 @@ class WarmStartNet {
                               : A == 2 ? conv3d_brick_kernel<2> : conv3d_brick_kernel<1>;
                     MF3D_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBrickSmemMax));
                     const int cols = ((d.nx + 8 * A - 1) / (8 * A)) * ((d.ny + 15) / 16);
-                    const int nzc = std::max(1, std::min(std::max(1, d.nz / 4), (2 * num_sms() + cols - 1) / cols));
                     BrickArgs g{};
                     g.A = A;
                     g.NP = NP;
                     g.coutp = coutp;
-                    g.zchunk = (d.nz + nzc - 1) / nzc;
+                    g.zchunk = brick_zchunk(cols, d.nz, num_sms());
                     const long long bricks = (long long)cols * ((d.nz + g.zchunk - 1) / g.zchunk);
                     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(bricks, num_sms()));
                     for (int c = 0; c < split; ++c) {
@@ -240,24 +253,81 @@ class WarmStartNet {
         MF3D_LAUNCH_CK();
     }
 
+    // Launch shape of the weight gradient of one layer.
+    struct WgPlan {
+        int Q, tiles, ndt, coN, BY, BZ, stages, chunks;
+        size_t smem, part_floats; // weight and bias partials
+    };
+    static WgPlan wgrad_plan(const Dims& d, int cin, int cout) {
+        WgPlan p{};
+        const int nhg = cin / 8;
+        // Two voxel planes per product for 16 -> 16 channels (8 of a product's 16 regions used instead of
+        // 6, half the products); else every (dy, dx) in one CTA; else one dy per CTA, over the widest
+        // share of the output channels whose accumulators fit (the activations are staged again for
+        // each share).
+        p.Q = 4 * nhg <= 16 && 18 * cout <= WG_COLS ? 2 : 1;
+        p.tiles = ((p.Q + 2) * nhg + 15) / 16;
+        p.ndt = 9;
+        p.coN = cout;
+        if (9 * p.tiles * p.Q * cout > WG_COLS) {
+            p.ndt = 3;
+            for (p.coN = cout; p.coN > 16 && (cout % p.coN || 3 * p.tiles * p.coN > WG_COLS); p.coN -= 16) {}
+        }
+        // the largest brick of which two fit in shared memory (halo rows and planes are staged again
+        // by the neighbouring bricks)
+        static const int shapes[7][2] = {{8, 6}, {8, 4}, {8, 2}, {4, 4}, {4, 2}, {2, 2}, {2, 1}};
+        for (const auto& sh : shapes) {
+            p.BY = sh[0];
+            p.BZ = sh[1];
+            if (p.BZ % p.Q) continue;
+            p.stages = 2;
+            p.smem = wg_smem(cin, p.coN, p.Q, p.tiles, p.BY, p.BZ, 2);
+            if (p.smem <= kBrickSmemMax) break;
+        }
+        if (p.smem > kBrickSmemMax) {
+            p.stages = 1;
+            p.smem = wg_smem(cin, p.coN, p.Q, p.tiles, p.BY, p.BZ, 1);
+        }
+        const int blocks = ((d.nx + WG_BX - 1) / WG_BX) * ((d.ny + p.BY - 1) / p.BY) * ((d.nz + p.BZ - 1) / p.BZ);
+        const int share = (9 / p.ndt) * (cout / p.coN); // CTAs that read the same bricks
+        p.chunks = std::max(1, std::min(blocks, num_sms() / share));
+        p.part_floats = (size_t)p.chunks * p.Q * cout * 27 * cin + (size_t)p.chunks * cout;
+        return p;
+    }
+
     // dW (FP32, [cout][27][cin]) and db ([cout]) of a convolution from its input x and the
-    // gradient dy of its pre-activation output; accumulate adds to dw / db
+    // gradient dy of its pre-activation output; accumulate adds to dw / db.  part: the partials,
+    // wgrad_plan().part_floats of them.
     static void wgrad(cudaStream_t s, const Dims& d, int cin, int cout, const __nv_bfloat16* x,
                       const __nv_bfloat16* dy, float* dw, float* db, float* part, size_t part_floats,
-                      int accumulate) {
-        const long long V = (long long)d.v();
-        int vpc = (int)std::max<long long>(WG_VOX, ((V + 63) / 64 + WG_VOX - 1) / WG_VOX * WG_VOX); // <= 64 chunks
-        int nch = (int)((V + vpc - 1) / vpc);
+                      int accumulate, int* err) {
+        if (cout * cin > 8192) throw Error(MF3D_E_INVALID, "layer too wide for the weight gradient");
+        const WgPlan p = wgrad_plan(d, cin, cout);
+        if (p.part_floats > part_floats) throw Error(MF3D_E_INVALID, "weight-gradient scratch too small");
         const size_t wn = (size_t)cout * 27 * cin;
-        if ((size_t)nch * wn > part_floats) throw Error(MF3D_E_INVALID, "weight-gradient scratch too small");
-        if (cout * cin > 2 * 16 * WG_NT) throw Error(MF3D_E_INVALID, "layer too wide for the weight gradient");
-        wgrad_kernel<<<dim3(27, nch), WG_NT, 0, s>>>(x, dy, part, d.nx, d.ny, d.nz, cin, cout, vpc);
+        WgArgs a{};
+        a.x = x;
+        a.dy = dy;
+        a.part = part;
+        a.bpart = part + (size_t)p.chunks * p.Q * wn;
+        a.nx = d.nx;
+        a.ny = d.ny;
+        a.nz = d.nz;
+        a.cin = cin;
+        a.cout = cout;
+        a.Q = p.Q;
+        a.tiles = p.tiles;
+        a.coN = p.coN;
+        a.BY = p.BY;
+        a.BZ = p.BZ;
+        a.stages = p.stages;
+        a.err = err;
+        auto kern = p.ndt == 9 ? wgrad_tc_kernel<9> : wgrad_tc_kernel<3>;
+        MF3D_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBrickSmemMax));
+        kern<<<dim3(p.chunks, 9 / p.ndt, cout / p.coN), WG_NT, p.smem, s>>>(a);
         MF3D_LAUNCH_CK();
-        wgrad_reduce_kernel<<<ew_grid(wn), 256, 0, s>>>(part, nch, wn, dw, accumulate);
-        MF3D_LAUNCH_CK();
-        bgrad_kernel<<<nch, 256, 0, s>>>(dy, part, V, cout, vpc);
-        MF3D_LAUNCH_CK();
-        wgrad_reduce_kernel<<<1, 256, 0, s>>>(part, nch, (size_t)cout, db, accumulate);
+        wgrad_reduce_kernel<<<(unsigned)((wn + 31) / 32 + (cout + 31) / 32), dim3(32, 8), 0, s>>>(
+            part, p.chunks * p.Q, wn, dw, a.bpart, p.chunks, cout, db, accumulate);
         MF3D_LAUNCH_CK();
     }
 
@@ -326,7 +396,10 @@ class WarmStartNet {
         bufs_.acc1 = f32(V1 * 32);
         bufs_.acc2 = f32(V2 * 64);
         bufs_.accc = f32(V1 * 64);
-        bufs_.part_floats = (size_t)64 * 27 * 128 * 64; // 64 chunks of the widest layer
+        bufs_.part_floats = 0; // the largest layer's weight-gradient partials
+        Dims dl[4] = {d, d.half(), d.half().half(), d.half().half().half()};
+        for (const LayerSpec& L : kLayers)
+            bufs_.part_floats = std::max(bufs_.part_floats, wgrad_plan(dl[L.level], L.cin, L.cout).part_floats);
         bufs_.part = f32(bufs_.part_floats);
         bufs_.d = d;
     }
@@ -377,7 +450,8 @@ class WarmStartNet {
         conv(s, d, kLayers[l].cout, kLayers[l].cin, g, WT(l), nullptr, 0, mask, 0, dx, err_.as<int>());
     }
     void wg(cudaStream_t s, int l, const Dims& d, const __nv_bfloat16* x, const __nv_bfloat16* g) {
-        wgrad(s, d, kLayers[l].cin, kLayers[l].cout, x, g, GW(l), GB(l), bufs_.part, bufs_.part_floats, 1);
+        wgrad(s, d, kLayers[l].cin, kLayers[l].cout, x, g, GW(l), GB(l), bufs_.part, bufs_.part_floats, 1,
+              err_.as<int>());
     }
 
     void backward(const Dims& d0, cudaStream_t s) {
@@ -650,11 +724,20 @@ int mf3d_nn_conv3d_wgrad(const mf3d_grid* g, int cin, int cout, const void* x, c
         check_grid(g);
         if (cin % 16 || cout % 16 || cin > nn::CONV_MAXC || cout > nn::CONV_MAXC)
             throw Error(MF3D_E_INVALID, "convolution channels must be multiples of 16 in [16, 128]");
-        const size_t part = (size_t)64 * 27 * cin * cout + (size_t)64 * cout;
+        if (cin < 16 || cout < 16) throw Error(MF3D_E_INVALID, "convolution channels must be multiples of 16 in [16, 128]");
+        const nn::Dims d{g->nx, g->ny, g->nz};
+        const size_t part = nn::WarmStartNet::wgrad_plan(d, cin, cout).part_floats;
         DevMem scratch(part * sizeof(float));
-        nn::WarmStartNet::wgrad((cudaStream_t)stream, nn::Dims{g->nx, g->ny, g->nz}, cin, cout,
-                                (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, dw, db, scratch.as<float>(), part, 0);
+        int* err = ws_err_flag();
+        nn::WarmStartNet::wgrad((cudaStream_t)stream, d, cin, cout, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy,
+                                dw, db, scratch.as<float>(), part, 0, err);
+        int e = 0;
+        MF3D_CK(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
         MF3D_CK(cudaStreamSynchronize((cudaStream_t)stream));
+        if (e) {
+            MF3D_CK(cudaMemset(err, 0, sizeof(int)));
+            throw Error(MF3D_E_CUDA, "a tensor-core pipeline wait timed out");
+        }
     });
 }
 

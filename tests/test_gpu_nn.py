@@ -88,6 +88,26 @@ def test_conv3d_weight_gradient_vs_oracle(mf3d, cin, cout):
     assert _rel(_np(db), rb) < 1e-5
 
 
+# one channel pair per launch shape of the weight gradient: three planes a product; every (dy, dx) in
+# a CTA with one and two M tiles; one dy per CTA with one, two and three tiles; a share of the output
+# channels per CTA; eight output groups that do not divide the CTA; on grids with ragged bricks
+@pytest.mark.parametrize("shape", [(8, 8, 16), (7, 9, 21), (13, 5, 8), (1, 1, 1), (20, 17, 34)])
+@pytest.mark.parametrize("cin,cout", [(16, 16), (32, 16), (32, 32), (16, 64), (64, 64), (96, 32), (112, 64), (32, 96),
+                                      (64, 128)])
+def test_conv3d_weight_gradient_launch_shapes(mf3d, shape, cin, cout):
+    """Products of BF16 values are exact in FP32 and a partial sum has at most a few hundred terms
+    here, so FP32 accumulation stays within a few 2^-24 of the largest term's sum: 1e-5."""
+    M = mf3d
+    r = np.random.default_rng(cin * 131 + cout + sum(shape))
+    nz, ny, nx = shape
+    x = _bf(r.normal(size=(nz * ny * nx, cin)))
+    dy = _bf(r.normal(size=(nz * ny * nx, cout)))
+    dw, db = M.nn_conv3d_wgrad(M.Grid3D(nx, ny, nz, 1.0), x, dy)
+    rw, rb = N.conv3d_wgrad(_np(x).reshape(nz, ny, nx, cin), _np(dy).reshape(nz, ny, nx, cout))
+    assert _rel(_np(dw), rw) < 1e-5
+    assert _rel(_np(db), rb) < 1e-5
+
+
 def _sample(M, n, seed, sigma2=1.0, lam=4.0):
     """(lnK, h) of one solver-generated pair on an n^3 grid, FP32 CUDA tensors."""
     import torch
