@@ -125,6 +125,45 @@ struct DevMem {
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
+// Scratch of one call, in stream order, from a pool of this library: cudaMalloc and cudaFree cost a call
+// 0.6 ms (they synchronise the device).  The pool keeps at most kScratchKeep bytes between calls and is
+// the driver's own, so calls on several threads and streams may use it at once.
+static constexpr unsigned long long kScratchKeep = 64ull << 20;
+static cudaMemPool_t scratch_pool() {
+    constexpr int kDevices = 64;
+    static std::mutex mu;
+    static cudaMemPool_t pools[kDevices] = {};
+    int dev = 0;
+    MF3D_CK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kDevices) throw Error(MF3D_E_INVALID, "device ordinal out of range for the scratch pool");
+    std::lock_guard<std::mutex> lock(mu);
+    if (!pools[dev]) {
+        cudaMemPoolProps pr{};
+        pr.allocType = cudaMemAllocationTypePinned;
+        pr.location.type = cudaMemLocationTypeDevice;
+        pr.location.id = dev;
+        cudaMemPool_t p;
+        MF3D_CK(cudaMemPoolCreate(&p, &pr));
+        unsigned long long keep = kScratchKeep;
+        MF3D_CK(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+        pools[dev] = p;
+    }
+    return pools[dev];
+}
+struct StreamMem {
+    void* p = nullptr;
+    cudaStream_t s;
+    StreamMem(size_t bytes, cudaStream_t stream) : s(stream) {
+        if (bytes) MF3D_CK(cudaMallocFromPoolAsync(&p, bytes, scratch_pool(), s));
+    }
+    ~StreamMem() {
+        if (p) cudaFreeAsync(p, s);
+    }
+    StreamMem(const StreamMem&) = delete;
+    StreamMem& operator=(const StreamMem&) = delete;
+    template <class T> T* as() const { return static_cast<T*>(p); }
+};
+
 static BcDev to_dev(const mf3d_bc& bc) {
     BcDev d;
     for (int f = 0; f < 6; ++f) {
@@ -1960,21 +1999,21 @@ static void run_velocity(const mf3d_grid* g, const mf3d_bc* bc, const double* h,
     VelOut o{U, V, W, layout};
     if (!out_host) {
         const ColLaunch cl = col_launch(g->nx, g->ny, g->nz);
-        velocity_kernel<<<cl.grid, cl.block, 0, s>>>(g->nx, g->ny, g->nz, g->dx, h, K, to_dev(*bc), o, nullptr, nullptr,
-                                                     nullptr, nullptr, cl.zchunk);
+        velocity_kernel<false><<<cl.grid, cl.block, 0, s>>>(g->nx, g->ny, g->nz, g->dx, h, K, to_dev(*bc), o, nullptr,
+                                                            nullptr, nullptr, nullptr, cl.zchunk);
         MF3D_LAUNCH_CK();
         return;
     }
     const ColLaunch cl = col_launch(g->nx, g->ny, g->nz);
     const unsigned nb = cl.nblocks;
-    DevMem scratch((size_t)nb * 2 * sizeof(double) + 64);
+    StreamMem scratch((size_t)nb * 2 * sizeof(double) + 64, s);
     char* base = scratch.as<char>();
     unsigned long long* mx = (unsigned long long*)base;
     unsigned* ticket = (unsigned*)(base + 8);
     double* sums = (double*)(base + 16);
     double* partials = (double*)(base + 64);
     MF3D_CK(cudaMemsetAsync(base, 0, 64, s));
-    velocity_kernel<<<cl.grid, cl.block, 0, s>>>(g->nx, g->ny, g->nz, g->dx, h, K, to_dev(*bc), o, mx, partials, ticket,
+    velocity_kernel<true><<<cl.grid, cl.block, 0, s>>>(g->nx, g->ny, g->nz, g->dx, h, K, to_dev(*bc), o, mx, partials, ticket,
                                                  sums, cl.zchunk);
     MF3D_LAUNCH_CK();
     unsigned long long hb[4];
@@ -2013,7 +2052,7 @@ int mf3d_velocity_diagnostics(const mf3d_grid* g, int layout, const double* U, c
         cudaStream_t s = (cudaStream_t)stream;
         const ColLaunch cl = col_launch(g->nx, g->ny, g->nz);
         // temporary reduction scratch, as the reference's compute_field_stats allocates its own
-        DevMem scr(stats_host ? (9 * (size_t)cl.nblocks + 16) * sizeof(double) : 0);
+        StreamMem scr(stats_host ? (9 * (size_t)cl.nblocks + 16) * sizeof(double) : 0, s);
         double* partials = stats_host ? scr.as<double>() : nullptr;
         double* stats_dev = stats_host ? partials + 9 * (size_t)cl.nblocks : nullptr;
         unsigned* ticket = stats_host ? reinterpret_cast<unsigned*>(stats_dev + 9) : nullptr;
@@ -2087,7 +2126,7 @@ int mf3d_velocity_mass_balance_noalloc(const mf3d_grid* g, const mf3d_bc* bc, co
         // max bits, ticket and sums must start at zero; the partials are written before read
         MF3D_CK(cudaMemsetAsync(base, 0, kMbNoAllocHeader, s));
         VelOut o{U, V, W, MF3D_VEL_COMPACT};
-        velocity_kernel<<<cl.grid, cl.block, 0, s>>>(g->nx, g->ny, g->nz, g->dx, h, K, to_dev(*bc), o, mx, partials,
+        velocity_kernel<true><<<cl.grid, cl.block, 0, s>>>(g->nx, g->ny, g->nz, g->dx, h, K, to_dev(*bc), o, mx, partials,
                                                      ticket, sums, cl.zchunk);
         MF3D_LAUNCH_CK();
         unsigned long long hb[4];
@@ -2363,6 +2402,39 @@ int mf3d_kfield_modes(unsigned long long seed, int n_modes, int cov, double lx, 
     });
 }
 
+// The modes of one part, in batches whose tables take at most `table` bytes (or 8 modes).
+static void kfield_part(KfPart w, double dx, int n_modes, const double* modes, double scale, double log_kg,
+                        int want_exp, double* out, size_t table, cudaStream_t s) {
+    const int nxp = (w.nx + 63) / 64 * 64;
+    const size_t nrows = (size_t)w.ny * w.nz, per = 2 * sizeof(double) * ((size_t)nxp + w.ny + w.nz);
+    const int all = (n_modes + KF_MC - 1) / KF_MC * KF_MC;
+    const int batch = (int)std::max<size_t>(KF_MC, std::min<size_t>(all, table / per / KF_MC * KF_MC));
+    StreamMem tab((size_t)batch * per, s);
+    double* tx = tab.as<double>();
+    double2* ty = reinterpret_cast<double2*>(tx + (size_t)batch * 2 * nxp);
+    double2* uv = ty + (size_t)batch * w.ny;
+    for (w.m0 = 0; w.m0 < n_modes; w.m0 += batch) {
+        w.n = std::min(batch, n_modes - w.m0);
+        w.last = w.m0 + w.n == n_modes;
+        const int mp = (w.n + KF_MC - 1) / KF_MC * KF_MC;
+        kfield_tables_kernel<<<grid1d((size_t)mp * (nxp + w.ny + w.nz), 256), 256, 0, s>>>(w, dx, n_modes, mp, nxp, modes,
+                                                                                          tx, ty, uv);
+        MF3D_LAUNCH_CK();
+        auto launch = [&](auto geom, auto kern) {
+            using KG = decltype(geom);
+            MF3D_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KG::SMEM));
+            const dim3 grid((unsigned)((nrows + KG::ROWS - 1) / KG::ROWS), (unsigned)((w.nx + KG::COLS - 1) / KG::COLS));
+            kern<<<grid, KF_NT, KG::SMEM, s>>>(w, mp, nxp, tx, ty, uv, scale, log_kg, want_exp, out);
+            MF3D_LAUNCH_CK();
+        };
+        // 64 columns a CTA unless the last 32 of them lie past the row; small fields in tiles of 32 rows, so
+        // that every SM has one
+        if (nrows * nxp < (size_t)num_sms() * 64 * 64) launch(KfGeom<1, 4, 1>{}, kfield_kernel<1, 4, 1>);
+        else if ((w.nx + 31) / 32 % 2 == 0) launch(KfGeom<4, 2, 2>{}, kfield_kernel<4, 2, 2>);
+        else launch(KfGeom<4, 4, 1>{}, kfield_kernel<4, 4, 1>);
+    }
+}
+
 int mf3d_kfield_eval(const mf3d_grid* g, int n_modes, const double* modes, double sigma2, double log_kg,
                      int want_exp, double* out, void* stream) {
     return guard([&] {
@@ -2371,10 +2443,22 @@ int mf3d_kfield_eval(const mf3d_grid* g, int n_modes, const double* modes, doubl
         need(out, "out");
         if (n_modes <= 0 || sigma2 < 0) throw Error(MF3D_E_INVALID, "bad n_modes or variance");
         cudaStream_t s = (cudaStream_t)stream;
-        const size_t tasks = (size_t)g->ny * g->nz * ((g->nx + KF_SEG - 1) / KF_SEG);
-        kfield_kernel<<<(unsigned)((tasks + KF_NT - 1) / KF_NT), KF_NT, 0, s>>>(
-            g->nx, g->ny, g->nz, g->dx, n_modes, modes, std::sqrt(sigma2), log_kg, want_exp, out);
-        MF3D_LAUNCH_CK();
+        const double scale = std::sqrt(sigma2) / std::sqrt((double)n_modes);
+        // one part in ordinary use; a very long axis or very many modes go in several, so that the tables stay
+        // below 256 MiB (or 8 modes)
+        constexpr int kAxis = 1 << 20;
+        constexpr size_t kTable = 256ull << 20;
+        KfPart w{};
+        w.NX = g->nx;
+        w.NY = g->ny;
+        for (w.oz = 0; w.oz < g->nz; w.oz += kAxis)
+            for (w.oy = 0; w.oy < g->ny; w.oy += kAxis)
+                for (w.ox = 0; w.ox < g->nx; w.ox += kAxis) {
+                    w.nx = std::min(kAxis, g->nx - w.ox);
+                    w.ny = std::min(kAxis, g->ny - w.oy);
+                    w.nz = std::min(kAxis, g->nz - w.oz);
+                    kfield_part(w, g->dx, n_modes, modes, scale, log_kg, want_exp, out, kTable, s);
+                }
         MF3D_CK(cudaStreamSynchronize(s));
     });
 }

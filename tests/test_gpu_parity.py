@@ -573,3 +573,80 @@ def test_bounded_mbarrier_waits_give_up_and_leave_the_context_usable(mf3d):
     s.set_K(_t(_lognormal((16, 16, 16), 1.0, 3)))
     res = s.solve(_t(np.zeros((16, 16, 16))))
     assert res.converged
+
+
+# the three tile shapes of the K generator (small fields; an even and an odd number of 32-cell column
+# blocks), ragged rows and columns, single rows and columns, a mode count that is no multiple of the batch
+@pytest.mark.parametrize("shape,modes", [((1, 1, 1), 1), ((3, 5, 31), 17), ((33, 40, 70), 100), ((90, 97, 64), 33),
+                                         ((60, 71, 160), 48), ((200, 120, 33), 20)])
+def test_kfield_tile_shapes_vs_oracle(mf3d, oracle_mod, shape, modes):
+    """Phases reach about 1e4 here, so a mode is off by at most a few 1e-12 of its amplitude."""
+    M, O = mf3d, oracle_mod
+    g = M.Grid3D(shape[2], shape[1], shape[0], 0.7)
+    table = M.kfield_modes(5, modes, M.COV_EXPONENTIAL, (4.0, 3.0, 2.0))
+    lnk = _np(M.generate_K_field(g, 1.5, (4.0, 3.0, 2.0), seed=5, n_modes=modes, log_only=True))
+    x = [(np.arange(n) + 0.5) * 0.7 for n in (shape[2], shape[1], shape[0])]
+    ref = np.zeros(shape)
+    for k1, k2, k3, a, b in table.T:
+        ph = (k3 * x[2])[:, None, None] + (k2 * x[1])[None, :, None] + (k1 * x[0])[None, None, :]
+        ref += a * np.sin(ph) + b * np.cos(ph)
+    ref *= np.sqrt(1.5 / modes)
+    assert np.abs(lnk - ref).max() < 1e-10
+    K = _np(M.generate_K_field(g, 1.5, (4.0, 3.0, 2.0), seed=5, n_modes=modes, K_geo=2.0))
+    assert np.allclose(K, 2.0 * np.exp(ref), rtol=1e-9)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 3, 2), (5, 1, 33), (7, 9, 32), (6, 17, 65), (40, 8, 31)])
+@pytest.mark.parametrize("per", [False, True])
+def test_velocity_and_diagnostics_edges_vs_numpy(mf3d, shape, per):
+    """Padded velocities and their diagnostics on tiles of one cell to ragged ones, against numpy's
+    evaluation of the same formulas (a handful of roundings: 1e-13 of each field's largest value)."""
+    M = mf3d
+    nz, ny, nx = shape
+    r = np.random.default_rng(nx + 10 * ny + 100 * nz)
+    K, h, dx = np.exp(r.normal(size=shape)), r.normal(size=shape), 0.5
+    faces = [M.BCFace(M.DIRICHLET, 1.0), M.BCFace(M.DIRICHLET, -0.5)]
+    bc = M.BCSpec(faces + [M.BCFace(M.PERIODIC if per else M.NEUMANN, 0.0) for _ in range(4)])
+    g = M.Grid3D(nx, ny, nz, dx)
+    bufs = [_t(np.zeros(n)) for n in M.velocity_sizes(g, M.VEL_PADDED)]
+    M.compute_velocity_from_head(*bufs, _t(h), _t(K), g, bc, M.VEL_PADDED)
+
+    def flux(a, b, ha, hb):
+        return 2.0 * a * b * (ha - hb) / ((a + b) * dx)
+
+    ref = []
+    for ax in (2, 1, 0):
+        n = shape[ax]
+        t = lambda v, lo, hi: np.take(v, np.arange(lo, hi), ax)  # noqa: E731
+        q = flux(t(K, 0, n - 1), t(K, 1, n), t(h, 0, n - 1), t(h, 1, n))
+        K0, K1, h0, h1 = t(K, 0, 1), t(K, n - 1, n), t(h, 0, 1), t(h, n - 1, n)
+        if ax == 2:
+            lo, hi = -K0 * (h0 - 1.0) / (dx / 2), -K1 * (-0.5 - h1) / (dx / 2)
+        else:
+            lo = hi = flux(K1, K0, h1, h0) if per else np.zeros_like(K0)
+        ref.append(np.concatenate([lo, q, hi], ax))
+    got = [_np(b).reshape(nz + 1, ny + 1, nx + 1) for b in bufs]
+    for a, o in zip(got, ref):
+        assert np.abs(a[:o.shape[0], :o.shape[1], :o.shape[2]] - o).max() <= 1e-13 * max(np.abs(o).max(), 1.0)
+    u, v, w = ref
+    div = ((u[..., 1:] - u[..., :-1]) + (v[:, 1:] - v[:, :-1]) + (w[1:] - w[:-1])) / dx
+    om, he = np.zeros(shape), np.zeros(shape)
+    if min(shape) >= 3:
+        c = [0.5 * (u[..., 1:] + u[..., :-1]), 0.5 * (v[:, 1:] + v[:, :-1]), 0.5 * (w[1:] + w[:-1])]
+        i = (slice(1, -1),) * 3
+
+        def d(a, ax):
+            s = [slice(1, -1)] * 3
+            lo, hi = list(s), list(s)
+            lo[ax], hi[ax] = slice(0, -2), slice(2, None)
+            return (a[tuple(hi)] - a[tuple(lo)]) * (0.5 / dx)
+
+        ox, oy, oz = d(c[2], 1) - d(c[1], 0), d(c[0], 0) - d(c[2], 2), d(c[1], 2) - d(c[0], 1)
+        om[i] = np.sqrt(ox ** 2 + oy ** 2 + oz ** 2)
+        he[i] = c[0][i] * ox + c[1][i] * oy + c[2][i] * oz
+    out = [_t(np.full(shape, np.nan)) for _ in range(3)]
+    st = M.velocity_diagnostics(*bufs, g, M.VEL_PADDED, *out)
+    for a, o, s in zip(out, (div, om, he), (st["div"], st["vorticity_mag"], st["helicity"])):
+        scale = max(np.abs(o).max(), np.abs(u).max() / dx)
+        assert np.abs(_np(a) - o).max() <= 1e-13 * max(scale, scale ** 2)
+        assert np.allclose(s, (o.min(), o.max(), o.mean()), rtol=1e-11, atol=1e-11 * max(scale, scale ** 2))
