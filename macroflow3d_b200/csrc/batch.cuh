@@ -68,9 +68,14 @@ struct Blob {
         if (src && bytes) std::memcpy(h.data() + off, src, bytes);
         return off;
     }
-    std::unique_ptr<DevMem> upload() const {
+    // on the stream that the table's readers run on: a copy on the legacy stream is not ordered before
+    // kernels of a non-blocking stream, and returns once the source is staged
+    std::unique_ptr<DevMem> upload(cudaStream_t s) const {
         std::unique_ptr<DevMem> m(new DevMem(std::max<size_t>(h.size(), 256)));
-        if (!h.empty()) MF3D_CK(cudaMemcpy(m->p, h.data(), h.size(), cudaMemcpyHostToDevice));
+        if (!h.empty()) {
+            MF3D_CK(cudaMemcpyAsync(m->p, h.data(), h.size(), cudaMemcpyHostToDevice, s));
+            MF3D_CK(cudaStreamSynchronize(s));
+        }
         return m;
     }
 };
@@ -207,7 +212,7 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
             }
             Blob b;
             b.add(items.data(), items.size() * sizeof(items[0]));
-            tail_mem_ = b.upload();
+            tail_mem_ = b.upload(s_);
             // largest tail of any batch (the attribute is the kernel's, shared by all batches)
             MF3D_CK(cudaFuncSetAttribute(tail2_batch_kernel<T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kTailSmemMax));
@@ -233,12 +238,14 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
                 it.tickets = H.tickets_.as<unsigned>();
                 it.err = H.err_.as<int>();
                 it.n = H.G_[0].n;
-                const ColLaunch cl = col_launch(H.G_[0].nx, H.G_[0].ny, H.G_[0].nz);
+                // blocks enough for the whole batch, not for each realisation alone: a block of a few
+                // planes stages two or three more, and a block of a few cells is all reduction
+                const ColLaunch cl = col_launch(H.G_[0].nx, H.G_[0].ny, H.G_[0].nz, std::max(1, std::min(8, 16 / R)));
                 it.zchunk = cl.zchunk;
                 it.cgx = (int)cl.grid.x;
                 it.cgy = (int)cl.grid.y;
                 it.cgz = (int)cl.grid.z;
-                it.n1 = (int)grid1d(it.n, PK_NT);
+                it.n1 = (int)std::max<size_t>(1, std::min<size_t>(grid1d(it.n, PK_NT), it.n / (8 * PK_NT)));
                 off3[r + 1] = off3[r] + (int)cl.nblocks;
                 off1[r + 1] = off1[r] + it.n1;
             }
@@ -251,7 +258,7 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
             const size_t oc = b.add(nullptr, 2 * R * sizeof(CopyItem));
             const size_t ost = b.add(nullptr, R * (sizeof(PcgState) + sizeof(int))); // states, then error flags
             const size_t octl = b.add(nullptr, sizeof(BatchCtl) + 16);
-            pcg_mem_ = b.upload();
+            pcg_mem_ = b.upload(s_);
             unsigned char* base = pcg_mem_->as<unsigned char>();
             items_d_ = reinterpret_cast<PcgItem*>(base + oi);
             off3_d_ = reinterpret_cast<int*>(base + o3);
@@ -477,7 +484,7 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
             L.nseg = (int)items.size();
             L.total = off.back();
             L.grid = (unsigned)L.total;
-            L.mem = b.upload();
+            L.mem = b.upload(s_);
             unsigned char* base = L.mem->template as<unsigned char>();
             L.roff = reinterpret_cast<const int*>(base + oo);
             L.ritems = reinterpret_cast<const RrItem<T, TC>*>(base + oi);
@@ -519,7 +526,7 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
             L.pair = true;
             L.nseg = (int)ps.size();
             L.total = off.back();
-            L.mem = b.upload();
+            L.mem = b.upload(s_);
             unsigned char* base = L.mem->template as<unsigned char>();
             L.pa0.seg_off = reinterpret_cast<const int*>(base + oo);
             L.pa0.seg_args = reinterpret_cast<const SpArgs<T, TC>*>(base + oa);
@@ -557,7 +564,7 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
             L.tma = true;
             L.nseg = (int)ts.size();
             L.total = off.back();
-            L.mem = b.upload();
+            L.mem = b.upload(s_);
             unsigned char* base = L.mem->template as<unsigned char>();
             L.a0.seg_off = reinterpret_cast<const int*>(base + oo);
             L.a0.seg_args = reinterpret_cast<const TmaSweepArgs<T, TC>*>(base + oa);
@@ -595,7 +602,7 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
             L.nseg = (int)ls.size();
             L.total = off.back();
             L.grid = (unsigned)L.total;
-            L.mem = b.upload();
+            L.mem = b.upload(s_);
             unsigned char* base = L.mem->template as<unsigned char>();
             L.loff = reinterpret_cast<const int*>(base + oo);
             L.largs = reinterpret_cast<const SweepArgs<T, TC, T>*>(base + oa);
@@ -804,6 +811,183 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
     int pre_launches_ = 0, body_launches_ = 0, post_launches_ = 0;
 };
 
+// ---------------------------------------------------------------------------------------
+// An ensemble: the larger realisations are solved by their own single-solve graphs, kStreams of them at a
+// time, the smaller ones as one batch (above).
+//
+// A single solve's kernels move their bytes at up to twice the rate of the batched ones (x-pair sweeps,
+// coarse levels in a cluster), but on a grid of 64^3 to 160^3 cells each fills the device for part of its
+// time only: several solves side by side fill it.  Measured, 16 realisations with edges of 64 to 160
+// (19.4 M cells): FP32 41.4 ms batched, 30.0 / 25.1 / 25.2 ms with 2 / 4 / 8 streams; FP64 89.8 ms, 34.7 / 30.2 /
+// 30.2 ms.  16 of 64^3: FP32 9.2 ms batched and 12.2 side by side, FP64 14.1 and 12.7; 16 of 32^3: 4.7 and 5.1, 5.7
+// and 5.0; 4 of 64^3: 4.3 and 3.2, 5.7 and 3.3; 4 of 48^3: 3.7 and 2.3.  Side by side a realisation costs 0.3 ms
+// and 1.3 ns a cell, in the batch 1.5 to 2 ns (FP32) or 2.5 to 4.4 ns (FP64) a cell after 3 to 4 ms for all.
+// ---------------------------------------------------------------------------------------
+class EnsembleSolver : public BatchSolverBase {
+  public:
+    static constexpr int kStreams = 4;
+    // realisations that are solved side by side: from this size on, and all of them when the batch would
+    // hold no more than kStreams
+    static std::vector<char> choose(int count, const mf3d_grid* g, int precision) {
+        const double least = precision == MF3D_PREC_FP64 ? 110e3 : 300e3;
+        std::vector<char> solo(count);
+        int small = 0;
+        for (int r = 0; r < count; ++r) {
+            solo[r] = (double)g[r].nx * g[r].ny * g[r].nz >= least;
+            small += !solo[r];
+        }
+        if (small <= kStreams) solo.assign(count, 1);
+        return solo;
+    }
+
+    // solo[i] is realisation solo_at[i]; batch (may be null) holds the realisations batch_at
+    EnsembleSolver(std::vector<std::unique_ptr<HeadSolver>>&& solo, std::vector<int> solo_at,
+                   std::unique_ptr<BatchSolverBase> batch, std::vector<int> batch_at, const mf3d_solver_config& cfg,
+                   cudaStream_t s, cudaStream_t own)
+        : solo_(std::move(solo)), solo_at_(std::move(solo_at)), batch_(std::move(batch)),
+          batch_at_(std::move(batch_at)), cfg_(cfg), s_(s), own_stream_(own) {
+        // the largest first, each to the stream with the fewest cells so far
+        order_.resize(solo_.size());
+        for (size_t i = 0; i < order_.size(); ++i) order_[i] = (int)i;
+        std::stable_sort(order_.begin(), order_.end(),
+                         [&](int a, int b) { return solo_[a]->G_[0].n > solo_[b]->G_[0].n; });
+        const int ns = std::max(1, std::min<int>(kStreams, (int)solo_.size()));
+        lanes_.resize(ns);
+        lane_of_.resize(solo_.size());
+        std::vector<size_t> load(ns, 0);
+        for (int i : order_) {
+            const int l = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+            lane_of_[i] = l;
+            load[l] += solo_[i]->G_[0].n + 400000; // (and the launches of its coarse levels)
+        }
+        try {
+            MF3D_CK(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
+            MF3D_CK(cudaEventCreate(&ev0_));
+            MF3D_CK(cudaEventCreate(&ev1_));
+            for (Lane& l : lanes_) {
+                MF3D_CK(cudaStreamCreateWithFlags(&l.s, cudaStreamNonBlocking));
+                MF3D_CK(cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming));
+            }
+        } catch (...) {
+            release();
+            throw;
+        }
+    }
+    ~EnsembleSolver() override {
+        for (Lane& l : lanes_)
+            if (l.s) cudaStreamSynchronize(l.s);
+        if (own_stream_) cudaStreamSynchronize(own_stream_);
+        solo_.clear();
+        batch_.reset();
+        release();
+        if (own_stream_) cudaStreamDestroy(own_stream_);
+    }
+
+    int count() const override { return (int)(solo_.size() + batch_at_.size()); }
+    long long device_bytes() const override {
+        long long b = batch_ ? batch_->device_bytes() : 0;
+        for (const auto& h : solo_) b += h->device_bytes();
+        return b;
+    }
+    std::vector<mf3d_batch_tuning> autotune(int reps) override {
+        return batch_ ? batch_->autotune(reps) : std::vector<mf3d_batch_tuning>();
+    }
+
+    void set_K(const double* const* K) override {
+        if (batch_) {
+            std::vector<const double*> kb;
+            for (int r : batch_at_) kb.push_back(K[r]);
+            batch_->set_K(kb.data());
+        }
+        on_lanes([&](int i, cudaStream_t s) { solo_[i]->set_K(K[solo_at_[i]], s); });
+    }
+
+    void solve(double* const* h, const double* const* x0, mf3d_solve_result* res) override {
+        for (size_t i = 0; i < solo_.size(); ++i) {
+            if (!solo_[i]->have_K_) throw Error(MF3D_E_STATE, "set_K must be called before solve");
+            if (!h[solo_at_[i]]) throw Error(MF3D_E_INVALID, "h is null");
+        }
+        std::vector<mf3d_solve_result> part(batch_at_.size());
+        const long long l0 = g_launches;
+        MF3D_CK(cudaEventRecord(ev0_, s_));
+        auto x0_of = [&](int r) { return x0 ? x0[r] : nullptr; };
+        if (cfg_.use_graph) {
+            on_lanes([&](int i, cudaStream_t s) { solo_[i]->enqueue(h[solo_at_[i]], x0_of(solo_at_[i]), s); });
+        } else { // (host-driven loops wait: one solve after the other)
+            for (size_t i = 0; i < solo_.size(); ++i) solo_[i]->enqueue(h[solo_at_[i]], x0_of(solo_at_[i]), s_);
+        }
+        MF3D_CK(cudaEventRecord(ev1_, s_));
+        if (batch_) {
+            std::vector<double*> hb;
+            std::vector<const double*> xb;
+            for (int r : batch_at_) {
+                hb.push_back(h[r]);
+                xb.push_back(x0_of(r));
+            }
+            batch_->solve(hb.data(), xb.data(), part.data());
+        }
+        MF3D_CK(cudaStreamSynchronize(s_));
+        float ms = 0.f;
+        MF3D_CK(cudaEventElapsedTime(&ms, ev0_, ev1_));
+        long long launches = g_launches - l0;
+        std::vector<mf3d_solve_result> own(solo_.size());
+        for (size_t i = 0; i < solo_.size(); ++i) {
+            solo_[i]->finish(&own[i]);
+            launches += own[i].kernel_launches - solo_[i]->launches_;
+        }
+        if (!part.empty()) {
+            ms += part[0].device_ms;
+            launches += part[0].kernel_launches;
+        }
+        if (!res) return;
+        for (size_t i = 0; i < own.size(); ++i) res[solo_at_[i]] = own[i];
+        for (size_t i = 0; i < part.size(); ++i) res[batch_at_[i]] = part[i];
+        for (int r = 0; r < count(); ++r) { // of the whole ensemble
+            res[r].device_ms = ms;
+            res[r].kernel_launches = (int)launches;
+        }
+    }
+
+  private:
+    struct Lane {
+        cudaStream_t s = nullptr;
+        cudaEvent_t done = nullptr;
+    };
+    // f(i, stream) for every solo realisation, on the lanes' streams between what s_ held before and what
+    // comes after
+    template <class F> void on_lanes(F&& f) {
+        if (solo_.empty()) return;
+        MF3D_CK(cudaEventRecord(fork_, s_));
+        for (Lane& l : lanes_) MF3D_CK(cudaStreamWaitEvent(l.s, fork_, 0));
+        for (int i : order_) f(i, lanes_[lane_of_[i]].s);
+        for (Lane& l : lanes_) {
+            MF3D_CK(cudaEventRecord(l.done, l.s));
+            MF3D_CK(cudaStreamWaitEvent(s_, l.done, 0));
+        }
+    }
+    void release() {
+        for (Lane& l : lanes_) {
+            if (l.done) cudaEventDestroy(l.done);
+            if (l.s) cudaStreamDestroy(l.s);
+        }
+        lanes_.clear();
+        if (fork_) cudaEventDestroy(fork_);
+        if (ev0_) cudaEventDestroy(ev0_);
+        if (ev1_) cudaEventDestroy(ev1_);
+        fork_ = ev0_ = ev1_ = nullptr;
+    }
+
+    std::vector<std::unique_ptr<HeadSolver>> solo_;
+    std::vector<int> solo_at_;
+    std::unique_ptr<BatchSolverBase> batch_;
+    std::vector<int> batch_at_;
+    mf3d_solver_config cfg_;
+    cudaStream_t s_ = nullptr, own_stream_ = nullptr;
+    std::vector<int> order_, lane_of_;
+    std::vector<Lane> lanes_;
+    cudaEvent_t fork_ = nullptr, ev0_ = nullptr, ev1_ = nullptr;
+};
+
 } // namespace mf3d
 
 // =========================================================================================
@@ -835,17 +1019,27 @@ int mf3d_batch_create(int count, const mf3d_grid* grids, const mf3d_bc* bc, cons
             s = own;
         }
         try {
-            std::vector<std::unique_ptr<HeadSolver>> hs;
-            for (int r = 0; r < count; ++r) hs.emplace_back(new HeadSolver(grids[r], *bc, c, s));
+            std::vector<std::unique_ptr<HeadSolver>> solo, hs;
+            std::vector<int> solo_at, batch_at;
+            const std::vector<char> side = EnsembleSolver::choose(count, grids, c.precision);
+            for (int r = 0; r < count; ++r) {
+                const bool alone = side[r] != 0;
+                (alone ? solo : hs).emplace_back(new HeadSolver(grids[r], *bc, c, s));
+                (alone ? solo_at : batch_at).push_back(r);
+            }
+            std::unique_ptr<BatchSolverBase> small;
+            if (!hs.empty()) {
+                if (c.precision == MF3D_PREC_FP64)
+                    small.reset(new BatchSolverT<double, double>(std::move(hs), c, s, nullptr));
+                else if (c.precision == MF3D_PREC_FP32)
+                    small.reset(new BatchSolverT<float, float>(std::move(hs), c, s, nullptr));
+                else
+                    small.reset(new BatchSolverT<float, __nv_bfloat16>(std::move(hs), c, s, nullptr));
+            }
             std::unique_ptr<mf3d_batch> b(new mf3d_batch());
-            if (c.precision == MF3D_PREC_FP64)
-                b->impl.reset(new BatchSolverT<double, double>(std::move(hs), c, s, own));
-            else if (c.precision == MF3D_PREC_FP32)
-                b->impl.reset(new BatchSolverT<float, float>(std::move(hs), c, s, own));
-            else if (c.precision == MF3D_PREC_BF16)
-                b->impl.reset(new BatchSolverT<float, __nv_bfloat16>(std::move(hs), c, s, own));
-            else
-                throw Error(MF3D_E_INVALID, "unknown precision");
+            b->impl.reset(new EnsembleSolver(std::move(solo), std::move(solo_at), std::move(small), std::move(batch_at),
+                                             c, s, own));
+            own = nullptr; // (the ensemble's now)
             *out = b.release();
         } catch (...) {
             if (own) {

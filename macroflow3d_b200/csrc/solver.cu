@@ -1460,7 +1460,7 @@ class HeadSolver {
         bytes_ += z_.bytes;
         flexible_ = cfg.flexible < 0 ? (prec != MF3D_PREC_FP64) : (cfg.flexible != 0);
         host_state_ = nullptr;
-        MF3D_CK(cudaMallocHost(&host_state_, sizeof(PcgState)));
+        MF3D_CK(cudaMallocHost(&host_state_, sizeof(PcgState) + sizeof(int)));
         MF3D_CK(cudaEventCreate(&ev0_));
         MF3D_CK(cudaEventCreate(&ev1_));
         MF3D_CK(cudaStreamSynchronize(stream_));
@@ -1485,10 +1485,18 @@ class HeadSolver {
         if (ctas) *ctas = cplan_.Lc >= 0 ? cplan_.cn : 0;
     }
 
-    void set_K(const double* K) {
+    void set_K(const double* K) { set_K(K, stream_); }
+    void set_K(const double* K, cudaStream_t s) {
         if (!K) throw Error(MF3D_E_INVALID, "K is null");
         const long long l0 = g_launches;
-        cudaStream_t s = stream_;
+        enqueue(h, x0, stream_);
+        MF3D_CK(cudaStreamSynchronize(stream_));
+        finish(res);
+    }
+
+    // The whole solve on stream s, its state copied to the host at the end; with use_graph nothing here
+    // waits.  finish() after the stream has been waited for.
+    void enqueue(double* h, const double* x0, cudaStream_t s) {
         const int nl = (int)G_.size();
         MF3D_CK(cudaMemcpyAsync(Klev_[0]->p, K, G_[0].n * sizeof(double), cudaMemcpyDeviceToDevice, s));
         for (int l = 0; l + 1 < nl; ++l) {
@@ -1508,12 +1516,14 @@ class HeadSolver {
             rhs_guess_kernel<<<cl.grid, cl.block, 0, s>>>(G_[0].nx, G_[0].ny, G_[0].nz, G_[0].dx, Kp[0], to_dev(bc_),
                                                           b_.as<double>(), x0_.as<double>(), cl.zchunk);
         }
+class EnsembleSolver;
         MF3D_LAUNCH_CK();
         setup_launches_ = (int)(g_launches - l0);
         have_K_ = true;
     }
 
     int setup_launches() const { return setup_launches_; }
+    friend class EnsembleSolver;
     void set_budget_ns(unsigned long long ns) { budget_ns_ = ns; }
 
     void vcycle(const double* r, double* z) {
@@ -1547,10 +1557,9 @@ class HeadSolver {
     void solve(double* h, const double* x0, mf3d_solve_result* res) {
         if (!have_K_) throw Error(MF3D_E_STATE, "set_K must be called before solve");
         if (!h) throw Error(MF3D_E_INVALID, "h is null");
-        cudaStream_t s = stream_;
         const size_t n = G_[0].n;
         const long long l0 = g_launches;
-        long long body_runs = 0;
+        body_runs_ = 0;
         MF3D_CK(cudaEventRecord(ev0_, s));
         MF3D_CK(cudaMemcpyAsync(x_.p, x0 ? x0 : x0_.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
         MF3D_CK(cudaMemsetAsync(tickets_.p, 0, tickets_.bytes, s));
@@ -1563,13 +1572,13 @@ class HeadSolver {
         if (cfg_.use_graph) {
             if (!loop_exec_) build_loop_graph();
             MF3D_CK(cudaGraphLaunch(loop_exec_, s));
-            body_runs = -1; // known once the iteration count is back
+            body_runs_ = -1; // known once the iteration count is back
         } else {
             // host-driven loop: one iteration per launch sequence, stop flag polled each time
             const int cap = cfg_.solver == MF3D_SOLVER_MG ? cfg_.mg_max_cycles : cfg_.cg_max_iter;
             for (int it = 0; it < std::max(cap, 1); ++it) {
                 record_body(s, false);
-                ++body_runs;
+                ++body_runs_;
                 MF3D_CK(cudaMemcpyAsync(host_state_, state_.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
                 MF3D_CK(cudaStreamSynchronize(s));
                 if (host_state_->stop) break;
@@ -1579,11 +1588,15 @@ class HeadSolver {
         MF3D_CK(cudaMemcpyAsync(h, x_.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
         MF3D_CK(cudaEventRecord(ev1_, s));
         MF3D_CK(cudaMemcpyAsync(host_state_, state_.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
-        MF3D_CK(cudaStreamSynchronize(s));
-        check_err();
+        MF3D_CK(cudaMemcpyAsync(host_state_ + 1, err_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+        launches_ = g_launches - l0;
+    }
+
+    void finish(mf3d_solve_result* res) {
+        if (*reinterpret_cast<const int*>(host_state_ + 1)) check_err();
         const PcgState& st = *host_state_;
-        long long launches = g_launches - l0;
-        if (body_runs < 0) launches += (long long)std::max(st.iter, 1) * body_launches_;
+        long long launches = launches_;
+        if (body_runs_ < 0) launches += (long long)std::max(st.iter, 1) * body_launches_;
         if (res) {
             std::memset(res, 0, sizeof(*res));
             res->num_iterations = st.iter;
@@ -1760,7 +1773,8 @@ class HeadSolver {
     DevMem x_, b_, r_, p_, p2_, Ap_, x0_, z_; // p_, p2_: search directions, alternating by iteration
     DevMem partials_, tickets_, state_, mb_, err_, r32_;
     std::unique_ptr<VCycleBase> vc_;
-    PcgState* host_state_ = nullptr;
+    PcgState* host_state_ = nullptr; // pinned: the state, then the pipelines' error flag
+    long long body_runs_ = 0, launches_ = 0;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
     cudaGraph_t loop_graph_ = nullptr;
     cudaGraphExec_t loop_exec_ = nullptr;

@@ -215,6 +215,38 @@ def test_nonfinite_realisation_does_not_stop_the_others(mf3d):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_mixed_sizes_keep_their_places(mf3d, prec):
+    """Realisations large enough to be solved side by side among seven small ones that are batched:
+    every head, count and warm start belongs to its own realisation (compared with single solves, as
+    above)."""
+    import torch
+    M = mf3d
+    shapes = [(32, 32, 32), (96, 80, 64), (32, 40, 32), (40, 32, 32), (80, 64, 96), (32, 32, 40), (48, 32, 32),
+              (32, 48, 32), (32, 32, 48)]
+    grids = [M.Grid3D(*s) for s in shapes]
+    bc = M.BCSpec.darcy_x()
+    cfg = _cfg(M, getattr(M, "PREC_" + prec.upper()))
+    Ks = _fields(M, grids, seed=700)
+    ref = _single(M, grids, bc, cfg, Ks)
+    b, got, _ = _batch(M, grids, bc, cfg, Ks)
+    for (hr, rr), (hb, rb) in zip(ref, got):
+        assert rb.converged and abs(rb.num_iterations - rr.num_iterations) <= ITER_SLACK[prec]
+        assert rb.num_levels == rr.num_levels and _rel(hb, hr) < HEAD_TOL
+    x0s = [None] * len(grids)
+    for r in (0, 1, 7):
+        x0s[r] = torch.from_numpy(got[r][0]).cuda()
+    hs = [torch.empty_like(K) for K in Ks]
+    res = b.solve(hs, x0s)
+    for r, (h, one) in enumerate(zip(hs, res)):
+        if x0s[r] is not None:
+            assert one.num_iterations <= 1
+        else:
+            assert one.num_iterations == got[r][1].num_iterations
+            assert np.array_equal(h.cpu().numpy(), got[r][0])
+    b.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_batch_vs_oracle(mf3d, oracle_mod, prec):
     """Three uneven realisations (non-cubic coarse grids) solved as one batch, each against the
     FP64 oracle at the same tolerance (the realisation loop the batch replaces:
