@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "../../include/mf3d.h"
+#include "kernels_brick.cuh"
 #include "kernels_coarse.cuh"
 #include "kernels_kfield.cuh"
 #include "kernels_mg.cuh"
@@ -729,6 +730,12 @@ template <class T, class TC> class VCycle : public VCycleBase {
             tail_.post = post;
             tail_.coarse_iters = coarse;
             // weights of every level either coarse kernel serves: [Lw, coarsest)
+        // levels whose legs run in bricks (kernels_brick.cuh): two sweeps a leg, and few enough bricks
+        brick_.assign(Lt, 0);
+        for (int l = 0; l < Lt; ++l) {
+            const dim3 g = brick_grid(G[l]);
+            brick_[l] = pre == 2 && post == 2 && (long long)g.x * g.y * g.z <= (long long)kBrickWaves * num_sms();
+        }
             Lw_ = cp_.Lc >= 0 ? std::min(cp_.Lc, Lt) : Lt;
             size_t wtot = 0;
             for (int l = Lw_; l < nl; ++l) wtot += 8 * G[l].n;
@@ -784,6 +791,7 @@ template <class T, class TC> class VCycle : public VCycleBase {
             // not lower it under this one
             if (tail_smem_ > kTailSmemMax) throw Error(MF3D_E_INVALID, "coarse tail exceeds shared memory");
             MF3D_CK(cudaFuncSetAttribute(tail2_kernel<T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            plan_dense(nl);
                                          (int)kTailSmemMax));
             MF3D_CK(cudaFuncSetAttribute(tail2_kernel<double, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kTailSmemMax));
@@ -828,7 +836,11 @@ template <class T, class TC> class VCycle : public VCycleBase {
             MF3D_LAUNCH_CK();
             wo += 8 * G_[l].n;
         }
-        if (cmap_) { // the coarsest level's sweeps as a matrix, one column per cell
+        if (dense_) { // the cycle on the levels from D_ on as a matrix, one column per cell
+            MF3D_CK(cudaMemsetAsync(dense_->p, 0, dense_->bytes, s));
+            dense_map_kernel<<<dtail_.L[0].n, DN_NT, dtail_smem_, s>>>(dtail_, dense_ld_, dense_->as<double>());
+            MF3D_LAUNCH_CK();
+        } else if (cmap_) { // the coarsest level's sweeps as a matrix, one column per cell
             const int nl = (int)G_.size();
             const CLevel& C = cp_.a.L[cp_.a.nlev - 1];
             MF3D_CK(cudaMemsetAsync(cmap_->p, 0, cmap_->bytes, s));
@@ -860,6 +872,11 @@ template <class T, class TC> class VCycle : public VCycleBase {
                 // staged levels: the last pre-sweep, then the residual and its restriction in a
                 // kernel of their own (batched solves record the fused form)
                 const bool split = (mode & M_RESID) && (tma_[l] || pair_[l]) && split_resid_ && !rec_;
+            if (brick_[l] && !rec_) {
+                brick_leg(s, l, nullptr, (T*)xa_[l]->p, nullptr, bc_next, nullptr);
+                cur[l] = (const T*)xa_[l]->p;
+                continue;
+            }
                 sweep(s, l, c, out, nullptr, split ? nullptr : bc_next, split ? (mode & ~M_RESID) : mode, nullptr);
                 if (split) resid_restrict(s, l, out, bc_next);
                 c = out;
@@ -887,6 +904,12 @@ template <class T, class TC> class VCycle : public VCycleBase {
                 rec_sw_ = 2 * sw; // (2 sw + 1: the residual + restriction after it)
                 sweep(s, l, c, out, e, nullptr, mode, rho_out);
                 c = out;
+            if (brick_[l] && !rec_) {
+                T* out = l == 0 ? z : other(l, c);
+                brick_leg(s, l, c, out, e, nullptr, l == 0 ? rho_out : nullptr);
+                fin[l] = out;
+                continue;
+            }
             }
             if (post_ == 0) {
                 T* out = (l == 0) ? z : other(l, c);
@@ -904,7 +927,21 @@ template <class T, class TC> class VCycle : public VCycleBase {
         const int nl = (int)G_.size();
         out.push_back(timing("vcycle_total", tm.mean_ms(reps, [&] { run(tm.s, zv, rho_out); }), 0.0, 1));
         const int Lb = coarse_start();
-        if (Lb >= 1) {
+        for (int l = 0; l < Lb; ++l) {
+            if (!brick_[l]) continue;
+            char nm[40];
+            T* xa = (T*)xa_[l]->p;
+            T* xb = (T*)xb_[l]->p;
+            const T* e = l + 1 == Lb ? (const T*)coarse_out(z) : (const T*)xa_[l + 1]->p;
+            const double nn = (double)G_[l].n, et = sizeof(T), ec = sizeof(TC);
+            std::snprintf(nm, sizeof(nm), "brick_l%d_down", l);
+            out.push_back(timing(nm, tm.mean_ms(reps, [&] { brick_leg(tm.s, l, nullptr, xa, nullptr, (T*)bl_[l + 1]->p, nullptr); }),
+                                 (2.125 * et + 3.0 * ec) * nn, 1));
+            std::snprintf(nm, sizeof(nm), "brick_l%d_up", l);
+            out.push_back(timing(nm, tm.mean_ms(reps, [&] { brick_leg(tm.s, l, xa, l == 0 ? z : xb, e, nullptr, l == 0 ? rho_out : nullptr); }),
+                                 (3.125 * et + 3.0 * ec + (l == 0 ? 8.0 : 0.0)) * nn, 1));
+        }
+        if (Lb >= 1 && !brick_[0]) {
             const double n = (double)G_[0].n, et = sizeof(T), ec = sizeof(TC);
             const double coef = 3.0 * n * ec, nc = n / 8.0;
             T* xa = (T*)xa_[0]->p;
@@ -960,9 +997,10 @@ template <class T, class TC> class VCycle : public VCycleBase {
                                      3.0 * et * nn + 3.0 * nn * ec, pre_ + post_));
             }
         }
+                if (brick_[l]) continue;
         if (Lb < nl) {
             T* outp = coarse_out(z);
-            out.push_back(timing(cluster_on() ? "coarse_cluster" : "coarse_tail",
+            out.push_back(timing(dense_on() ? "coarse_bricks_matrix" : cluster_on() ? "coarse_cluster" : "coarse_tail",
                                  tm.mean_ms(reps, [&] { launch_tail(tm.s, outp); }), 0.0, 1));
         }
     }
@@ -982,7 +1020,121 @@ template <class T, class TC> class VCycle : public VCycleBase {
         const int Lb = coarse_start();
         if (Lb == 0) return z;
         if (cluster_on() && Lb < Lt_) return (T*)ctail_out_->p;
+    // Bricks of a level whose legs run in one launch each: up to kBrickWaves per SM.  A wave
+    // takes about 6.5 us a leg whatever the level, the five launches it replaces about 30 us on 32^3 to 64^3 cells
+    // (FP32: 48^3, 216 bricks, 31.5 us in bricks and 31 us as sweeps; 64^3, 512 bricks, 59 and 40 us; FP64:
+    // 48 x 32 x 48, 288 bricks, 27 and 32 us).
+    static constexpr int kBrickWaves = sizeof(T) == 4 ? 1 : 2;
+    static dim3 brick_grid(const Geom& g) {
+        constexpr int bz = BrickGeom<T>::BZ;
+        return dim3((unsigned)((g.nx + BK_B - 1) / BK_B), (unsigned)((g.ny + BK_B - 1) / BK_B), (unsigned)((g.nz + bz - 1) / bz));
+    }
+    // one leg of level l: down (x_in null) into x_out and b_coarse, or up from x_in and the correction e
+    void brick_leg(cudaStream_t s, int l, const T* x_in, T* x_out, const T* e, T* b_coarse, double* dot_out) {
+        BrickLegArgs<T, TC> a{};
+        a.L = ops_[l];
+        a.b = l == 0 ? b0_ : (const T*)bl_[l]->p;
+        a.x_in = x_in;
+        a.e_c = e;
+        a.ncx = G_[l + 1].nx;
+        a.ncy = G_[l + 1].ny;
+        a.x_out = x_out;
+        a.b_coarse = b_coarse;
+        a.r64 = r64_;
+        a.dot_partials = scr_.partials;
+        a.dot_ticket = scr_.tickets + 0;
+        a.dot_out = dot_out;
+        const dim3 g = brick_grid(G_[l]);
+        if (!x_in) brick_leg_kernel<T, TC, false, false><<<g, BK_NT, 0, s>>>(a);
+        else if (!dot_out) brick_leg_kernel<T, TC, true, false><<<g, BK_NT, 0, s>>>(a);
+        else brick_leg_kernel<T, TC, true, true><<<g, BK_NT, 0, s>>>(a);
+        MF3D_LAUNCH_CK();
+    }
+
         return (T*)tail_out_->p;
+    }
+
+    // ---- the FP64 levels of a single solve as bricks and one matrix ----
+    // The levels from the first FP64 one down to D_ (the first of at most DN_MAX cells, or the coarsest one of
+    // at most DN_MAX_LAST) run their legs in bricks, and the cycle from D_ on is a matrix product.  Where
+    // neither size fits, or other sweep counts need a level of legs, the cluster kernel or the one-CTA tail
+    // serves.
+    void plan_dense(int nl) {
+        const int Ls = cp_.Lc >= 0 ? cp_.Lc : Lt_;
+        if (std::getenv("MF3D_NO_CLUSTER_TAIL")) return;
+        int D = Ls;
+        while (D < nl && G_[D].n > (size_t)DN_MAX) ++D;
+        if (D == nl && G_[nl - 1].n <= (size_t)DN_MAX_LAST) D = nl - 1;
+        if (D == nl || D < Lt_ || (D > Ls && !(pre_ == 2 && post_ == 2))) return;
+        dtail_ = tail_;
+        dtail_.nlev = nl - D;
+        int off = 0;
+        for (int l = D; l < nl; ++l) {
+            TailLevel& L = dtail_.L[l - D];
+            L = tail_.L[l - Lt_];
+            L.xoff = off;
+            off += (L.nx + 2) * (L.ny + 2) * (L.nz + 2);
+            L.boff = off;
+            off += L.n;
+        }
+        dtail_smem_ = (size_t)off * sizeof(double);
+        if (dtail_smem_ > 100 * 1024) return;
+        MF3D_CK(cudaFuncSetAttribute(dense_map_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        const int n = (int)G_[D].n;
+        dense_ld_ = n + (n & 1);
+        dense_.reset(new DevMem((size_t)n * dense_ld_ * sizeof(double)));
+        bytes_ += dense_->bytes;
+        D_ = D;
+        size_t total = 0; // FP64 vectors: b, x (down leg) and x (up leg) of the levels Ls .. D
+        c64_.resize(nl);
+        for (int l = Ls; l <= D; ++l) total += 3 * G_[l].n;
+        dvec_.reset(new DevMem(total * sizeof(double)));
+        bytes_ += dvec_->bytes;
+        double* p = dvec_->as<double>();
+        for (int l = Ls; l <= D; ++l) {
+            c64_[l] = {p, p + G_[l].n, p + 2 * G_[l].n};
+            p += 3 * G_[l].n;
+        }
+    }
+    bool dense_on() const { return dense_ && !rec_tail_ && !rec_; }
+    template <class TB, class TO>
+    void coarse_leg(cudaStream_t s, int l, const TB* b, const double* x_in, const double* e, TO* x_out, double* b_coarse) {
+        BrickLegArgs<double, double, TB, TO> a{};
+        a.L = op64_[l];
+        a.b = b;
+        a.x_in = x_in;
+        a.e_c = e;
+        a.ncx = G_[l + 1].nx;
+        a.ncy = G_[l + 1].ny;
+        a.x_out = x_out;
+        a.b_coarse = b_coarse;
+        constexpr int bz = BrickGeom<double>::BZ;
+        const Geom& g = G_[l];
+        const dim3 grid((unsigned)((g.nx + BK_B - 1) / BK_B), (unsigned)((g.ny + BK_B - 1) / BK_B), (unsigned)((g.nz + bz - 1) / bz));
+        if (x_in) brick_leg_kernel<double, double, true, false, TB, TO><<<grid, BK_NT, 0, s>>>(a);
+        else brick_leg_kernel<double, double, false, false, TB, TO><<<grid, BK_NT, 0, s>>>(a);
+        MF3D_LAUNCH_CK();
+    }
+    // b_in: b of the first FP64 level
+    template <class TB> void dense_end(cudaStream_t s, const TB* b_in, T* out) {
+        const int Ls = coarse_start(), n = (int)G_[D_].n;
+        const double* M = dense_->as<double>();
+        const unsigned gd = (unsigned)((n + DA_NT / 32 - 1) / (DA_NT / 32));
+        if (D_ == Ls) {
+            dense_apply_kernel<TB, T><<<gd, DA_NT, 0, s>>>(n, dense_ld_, M, b_in, out);
+            MF3D_LAUNCH_CK();
+            return;
+        }
+        for (int l = Ls; l < D_; ++l) {
+            if (l == Ls) coarse_leg<TB, double>(s, l, b_in, nullptr, nullptr, c64_[l].x, c64_[l + 1].b);
+            else coarse_leg<double, double>(s, l, c64_[l].b, nullptr, nullptr, c64_[l].x, c64_[l + 1].b);
+        }
+        dense_apply_kernel<double, double><<<gd, DA_NT, 0, s>>>(n, dense_ld_, M, c64_[D_].b, c64_[D_].y);
+        MF3D_LAUNCH_CK();
+        for (int l = D_ - 1; l >= Ls; --l) {
+            if (l == Ls) coarse_leg<TB, T>(s, l, b_in, c64_[l].x, c64_[l + 1].y, out, nullptr);
+            else coarse_leg<double, double>(s, l, c64_[l].b, c64_[l].x, c64_[l + 1].y, c64_[l].y, nullptr);
+        }
     }
 
     void launch_tail(cudaStream_t s, T* out) {
@@ -994,6 +1146,11 @@ template <class T, class TC> class VCycle : public VCycleBase {
             return;
         }
         if (rec_tail_) { // batched solve: record only (the batch needs a level above the tail)
+        if (dense_on()) {
+            if (coarse_start() == 0) dense_end(s, r64_, out);
+            else dense_end(s, (const T*)bl_[coarse_start()]->p, out);
+            return;
+        }
             if (Lt_ == 0) throw Error(MF3D_E_INVALID, "batched solve: the whole hierarchy fits the coarse tail");
             rec_tail_->a = tail_;
             rec_tail_->b = (const T*)bl_[Lt_]->p;
@@ -1323,12 +1480,21 @@ template <class T, class TC> class VCycle : public VCycleBase {
     std::unique_ptr<DevMem> tail_out_, tail_w_, ctail_out_, cmap_;
     Tail2Args tail_{};
     int Lw_ = 0; // first level with FP64 weights
+    std::vector<int> brick_;   // levels whose legs run in bricks
     size_t tail_smem_ = 0;
     size_t bytes_ = 0;
 };
 
 template <class T>
 __global__ void dot_kernel(size_t n, const double* __restrict__ a, const T* __restrict__ b, double* partials,
+    struct Coarse64 {
+        double *b = nullptr, *x = nullptr, *y = nullptr;
+    };
+    std::unique_ptr<DevMem> dense_, dvec_; // the matrix of level D_; FP64 vectors of the levels above it
+    std::vector<Coarse64> c64_;
+    Tail2Args dtail_{};
+    int D_ = 0, dense_ld_ = 0;
+    size_t dtail_smem_ = 0;
                            unsigned* ticket, double* out) {
     double acc = 0.0;
     for (size_t c = blockIdx.x * (size_t)PK_NT + threadIdx.x; c < n; c += (size_t)gridDim.x * PK_NT)
