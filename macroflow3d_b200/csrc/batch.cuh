@@ -720,6 +720,8 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
 
     void record_post(cudaStream_t s) {
         const int R = (int)hs_.size();
+        batch_xfinish_kernel<<<pgrid(tot1_), PK_NT, 0, s>>>(items_d_, off1_d_, R, tot1_);
+        MF3D_LAUNCH_CK();
         batch_residual_kernel<<<pgrid(tot3_), dim3(32, 8), 0, s>>>(items_d_, off3_d_, R, tot3_, 1,
                                                                    cfg_.conv_norm == MF3D_CONV_B ? 1 : 0);
         MF3D_LAUNCH_CK();

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(PMV_TX * PMV_TY, MF3D_PMATVEC_MINB)
         const int s = find_seg(off, nseg, b);
         const PcgItem& it = items[s];
         const VBlk vb = make_vblk(b - __ldg(off + s), it.cgx, it.cgy, it.cgz);
-        pmatvec_body<TZ>(it.L, (const TZ*)it.z, it.p, it.p2, it.Ap, it.st, it.partials, it.tickets + 3, it.zchunk, vb,
+        pmatvec_body<TZ>(it.L, (const TZ*)it.z, it.p, it.p2, it.Ap, it.x, it.st, it.partials, it.tickets + 3, it.zchunk, vb,
                          bpmv_sm);
     }
 }
@@ -148,9 +148,18 @@ __global__ void __launch_bounds__(PK_NT) batch_xr_update_kernel(const PcgItem* _
         const PcgItem& it = items[s];
         if (it.st->stop) continue;
         const int o = __ldg(off + s);
-        const double* p = pcg_pbuf_out(it.st->iter, it.p, it.p2); // this iteration's direction
-        xr_update_body<TZ>(it.n, it.x, p, it.r, it.Ap, (const TZ*)it.z, it.st, it.partials, it.tickets + 4, 0, 0,
+        xr_update_body<TZ>(it.n, it.r, it.Ap, (const TZ*)it.z, it.st, it.partials, it.tickets + 4, 0, 0,
                            it.r32, b - o, __ldg(off + s + 1) - o);
+    }
+}
+
+// the steps that the heads do not hold yet, after the loop
+__global__ void __launch_bounds__(PK_NT) batch_xfinish_kernel(const PcgItem* __restrict__ items,
+                                                              const int* __restrict__ off, int nseg, int total) {
+    for (int b = blockIdx.x; b < total; b += gridDim.x) {
+        const int s = find_seg(off, nseg, b), o = __ldg(off + s);
+        const PcgItem& it = items[s];
+        xfinish_body(it.n, it.x, it.p, it.p2, it.st, b - o, __ldg(off + s + 1) - o);
     }
 }
 

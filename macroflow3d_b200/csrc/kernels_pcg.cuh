@@ -25,6 +25,8 @@ struct PcgState {
     double rtol;
     double final_res; // ||r|| at the last check
     double alpha, beta;
+    double alpha_prev; // the step before alpha
+    int x_done;        // steps that x holds (the others are added two at a time, see pmatvec_body)
     int iter, max_iter, check_every, flexible;
     int converged, status, stop, body_count;
     int solver;                    // MF3D_SOLVER_*: 0 PCG_MG, 1 standalone MG, 2 plain CG
@@ -120,7 +122,8 @@ __device__ __forceinline__ void residual_body(const LevelOp<TC>& L, const double
             st->converged = 0;
             st->status = PCG_OK;
             st->rho_new = st->rho_old = st->gamma = st->pAp = 0.0;
-            st->alpha = st->beta = 0.0;
+            st->alpha = st->alpha_prev = st->beta = 0.0;
+            st->x_done = 0;
             if (st->solver == SOLVE_MG) {
                 // mg_solve has no early exit (src/multigrid/cycle/v_cycle.cu:90-113)
                 st->stop = st->max_iter <= 0 ? 1 : 0;
@@ -174,7 +177,11 @@ __global__ void __launch_bounds__(PK_NT) residual_kernel(const LevelOp<TC> L, co
 // exactly; Fletcher-Reeves rho_new / rho_old, or the flexible Polak-Ribiere form
 // (rho_new - gamma) / rho_old) fused with Ap = A p and <p, Ap>: p_new is formed once per cell
 // from z and p_old and written once, instead of written by one kernel and re-read by the
-// next.  p_old and p_new live in two buffers that swap by iteration parity (pcg_pbuf_in /
+// next.  The head update is here too, two steps at a time: x += alpha_{k-2} p_{k-2} + alpha_{k-1} p_{k-1} in every
+// second iteration, where p_{k-1} is staged anyway and p_{k-2} is the value that p_k is about to replace.  x and
+// p cross the memory 12 bytes a cell and iteration instead of 24 in a pass with r; the sums are rounded in the
+// same order, so x is the same to the last bit.  xfinish_kernel adds what is left after the loop.
+// p_old and p_new live in two buffers that swap by iteration parity (pcg_pbuf_in /
 // pcg_pbuf_out): no CTA overwrites a value that another still reads.
 //
 // 2.5-D blocking: a CTA of 32 x 8 threads owns a 32 x 8 column tile and marches a z chunk.
@@ -227,8 +234,9 @@ template <int B> __device__ __forceinline__ void pmv_cp(void* dst, const void* s
 // the top.
 template <class TZ>
 __device__ __forceinline__ void pmatvec_body(const LevelOp<double>& L, const TZ* __restrict__ z, double* p0,
-                                             double* p1, double* __restrict__ Ap, PcgState* st, double* partials,
-                                             unsigned* ticket, int zchunk, const VBlk& vb, unsigned char* sm) {
+                                             double* p1, double* __restrict__ Ap, double* __restrict__ x, PcgState* st,
+                                             double* partials, unsigned* ticket, int zchunk, const VBlk& vb,
+                                             unsigned char* sm) {
     constexpr int W = PMV_TX + 2; // slab / staged-plane row pitch
     PmvSlot<TZ>* slot = reinterpret_cast<PmvSlot<TZ>*>(sm);
     double* slab = reinterpret_cast<double*>(sm + PMV_NS * sizeof(PmvSlot<TZ>)); // [2][PMV_TY + 2][W]
@@ -238,9 +246,13 @@ __device__ __forceinline__ void pmatvec_body(const LevelOp<double>& L, const TZ*
     const bool first = s.iter == 0;
     const double beta = first ? 0.0 : (s.rho_new - (s.flexible ? s.gamma : 0.0)) / s.rho_old;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    if (vb.id == 0 && tx == 0 && ty == 0) st->beta = beta;
+    const bool xup = s.iter >= 2 && (s.iter & 1) == 0; // x takes the two steps before this one
+    if (vb.id == 0 && tx == 0 && ty == 0) {
+        st->beta = beta;
+        if (xup) st->x_done = s.iter;
+    }
     const double* __restrict__ pin = pcg_pbuf_in(s.iter, p0, p1);
-    double* __restrict__ pout = pcg_pbuf_out(s.iter, p0, p1);
+    double* pout = pcg_pbuf_out(s.iter, p0, p1);
     const int nx = L.nx, ny = L.ny, nz = L.nz;
     const size_t nxy = (size_t)nx * ny;
     const int i0 = vb.x * PMV_TX, j0 = vb.y * PMV_TY, i = i0 + tx, j = j0 + ty;
@@ -345,6 +357,9 @@ __device__ __forceinline__ void pmatvec_body(const LevelOp<double>& L, const TZ*
     for (int q = 0; q < PMV_NS - 1; ++q) issue(k0 + q);
     asm volatile("cp.async.wait_group %0;" ::"n"(PMV_NS - 2) : "memory");
     double pc = form(slot[0], slab);
+    const bool xown = xup && own;
+    double xn = 0.0, p2n = 0.0; // x and p_{k-2} of the next plane
+    if (xown) xn = x[c], p2n = pout[c];
     for (int k = k0; k < k1; ++k, c += nxy) {
         // this thread's copies of plane k+1 have landed; the barrier publishes everyone's
         // copies of plane k and the slab of plane k, and frees the slot of plane k-1
@@ -365,6 +380,11 @@ __device__ __forceinline__ void pmatvec_body(const LevelOp<double>& L, const TZ*
             const double sum = cxp * pe + cxm * pw + cyp * pn + cym * ps + czp * pt + czm * pb;
             const double y = (sum - D * pc) * L.inv_dx2;
             Ap[c] = y;
+            if (xup) {
+                const double xa = xn + s.alpha_prev * p2n;
+                x[c] = xa + s.alpha * (&S.p[0][0])[fO];
+                if (k + 1 < k1) xn = x[c + nxy], p2n = pout[c + nxy];
+            }
             pout[c] = pc;
             acc += pc * y;
             czm = czp;
@@ -380,17 +400,36 @@ __device__ __forceinline__ void pmatvec_body(const LevelOp<double>& L, const TZ*
 template <class TZ>
 __global__ void __launch_bounds__(PMV_TX * PMV_TY, MF3D_PMATVEC_MINB)
     pmatvec_dot_kernel(const LevelOp<double> L, const TZ* __restrict__ z, double* p0, double* p1,
-                       double* __restrict__ Ap, PcgState* st, double* partials, unsigned* ticket, int zchunk) {
+                       double* __restrict__ Ap, double* __restrict__ x, PcgState* st, double* partials,
+                       unsigned* ticket, int zchunk) {
     extern __shared__ __align__(16) unsigned char pmv_sm[];
-    pmatvec_body<TZ>(L, z, p0, p1, Ap, st, partials, ticket, zchunk, hw_vblk(), pmv_sm);
+    pmatvec_body<TZ>(L, z, p0, p1, Ap, x, st, partials, ticket, zchunk, hw_vblk(), pmv_sm);
 }
 
-// x += alpha p; r -= alpha Ap (alpha = rho_new / pAp); ||r||^2 and, for the flexible form,
+// The steps that x does not hold yet (at most two, see pmatvec_body), after the loop.
+__device__ __forceinline__ void xfinish_body(size_t n, double* __restrict__ x, const double* __restrict__ p0,
+                                             const double* __restrict__ p1, const PcgState* st, int blk, int nblk) {
+    const int it = st->iter, left = it - st->x_done;
+    if (st->solver == SOLVE_MG || left < 1 || left > 2) return;
+    const double a1 = st->alpha, a0 = st->alpha_prev;
+    const double* pa = ((it - 1) & 1) ? p0 : p1; // p_{it-1}: pcg_pbuf_out(it - 1)
+    const double* pb = ((it - 1) & 1) ? p1 : p0; // p_{it-2}
+    for (size_t c = blk * (size_t)PK_NT + threadIdx.x; c < n; c += (size_t)nblk * PK_NT) {
+        double v = x[c];
+        if (left == 2) v = v + a0 * pb[c];
+        x[c] = v + a1 * pa[c];
+    }
+}
+__global__ void __launch_bounds__(PK_NT) xfinish_kernel(size_t n, double* __restrict__ x, const double* __restrict__ p0,
+                                                        const double* __restrict__ p1, const PcgState* st) {
+    xfinish_body(n, x, p0, p1, st, blockIdx.x, gridDim.x);
+}
+
+// r -= alpha Ap (alpha = rho_new / pAp); ||r||^2 and, for the flexible form,
 // gamma = <r_{k+1}, z_k>.  The last CTA runs the stopping test of pcg.cuh:156-164 and sets
 // the graph's while condition.
 template <class TZ>
-__device__ __forceinline__ void xr_update_body(size_t n, double* __restrict__ x, const double* __restrict__ p,
-                                               double* __restrict__ r, const double* __restrict__ Ap,
+__device__ __forceinline__ void xr_update_body(size_t n, double* __restrict__ r, const double* __restrict__ Ap,
                                                const TZ* __restrict__ z, PcgState* st, double* partials,
                                                unsigned* ticket, cudaGraphConditionalHandle cond, int use_cond,
                                                float* __restrict__ r32, int blk, int nblk) {
@@ -415,7 +454,6 @@ __device__ __forceinline__ void xr_update_body(size_t n, double* __restrict__ x,
     // two cells per thread and pass (16-byte loads and stores); the vectors come from whole
     // allocations, so a pair starts on a 16-byte boundary; an odd last cell goes to thread 0
     auto cell = [&](size_t c) {
-        x[c] = x[c] + alpha * p[c];
         const double rv = r[c] + (-alpha) * Ap[c];
         r[c] = rv;
         if (r32) r32[c] = (float)rv;
@@ -424,15 +462,10 @@ __device__ __forceinline__ void xr_update_body(size_t n, double* __restrict__ x,
     };
     const size_t n2 = n >> 1;
     for (size_t c2 = blk * (size_t)PK_NT + threadIdx.x; c2 < n2; c2 += (size_t)nblk * PK_NT) {
-        double2 xv = reinterpret_cast<const double2*>(x)[c2];
-        const double2 pv = reinterpret_cast<const double2*>(p)[c2];
         double2 rv = reinterpret_cast<const double2*>(r)[c2];
         const double2 av = reinterpret_cast<const double2*>(Ap)[c2];
-        xv.x = xv.x + alpha * pv.x;
-        xv.y = xv.y + alpha * pv.y;
         rv.x = rv.x + (-alpha) * av.x;
         rv.y = rv.y + (-alpha) * av.y;
-        reinterpret_cast<double2*>(x)[c2] = xv;
         reinterpret_cast<double2*>(r)[c2] = rv;
         if (r32) reinterpret_cast<float2*>(r32)[c2] = make_float2((float)rv.x, (float)rv.y);
         srr += rv.x * rv.x;
@@ -455,6 +488,7 @@ __device__ __forceinline__ void xr_update_body(size_t n, double* __restrict__ x,
     if (grid_sums<PK_NT, 2>(v, partials, ticket, nblk, out, blk)) {
         const int it = s.iter + 1;
         st->iter = it;
+        st->alpha_prev = s.alpha;
         st->alpha = alpha;
         st->rr = out[0];
         st->gamma = out[1];
@@ -487,16 +521,12 @@ __device__ __forceinline__ void xr_update_body(size_t n, double* __restrict__ x,
 }
 
 template <class TZ>
-__global__ void __launch_bounds__(PK_NT) xr_update_kernel(size_t n, double* __restrict__ x, const double* __restrict__ p,
-                                                          double* __restrict__ r, const double* __restrict__ Ap,
-                                                          const TZ* __restrict__ z, PcgState* st,
-                                                          double* partials, unsigned* ticket,
+__global__ void __launch_bounds__(PK_NT) xr_update_kernel(size_t n, double* __restrict__ r,
+                                                          const double* __restrict__ Ap, const TZ* __restrict__ z,
+                                                          PcgState* st, double* partials, unsigned* ticket,
                                                           cudaGraphConditionalHandle cond, int use_cond,
-                                                          float* __restrict__ r32, const double* p_alt) {
-    // p_alt: the second search-direction buffer of pmatvec_dot_kernel (p is then the first);
-    // this iteration's direction is the one that kernel wrote
-    if (p_alt) p = (st->iter & 1) ? p : p_alt;
-    xr_update_body<TZ>(n, x, p, r, Ap, z, st, partials, ticket, cond, use_cond, r32, blockIdx.x, gridDim.x);
+                                                          float* __restrict__ r32) {
+    xr_update_body<TZ>(n, r, Ap, z, st, partials, ticket, cond, use_cond, r32, blockIdx.x, gridDim.x);
 }
 
 // Sets the while condition before the loop from the state left by residual_kernel(mode 0).

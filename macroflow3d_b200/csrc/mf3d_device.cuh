@@ -123,28 +123,61 @@ __device__ __forceinline__ double block_sum(double v, double* red /* NT/32 doubl
 template <int NT, int NV>
 __device__ __forceinline__ bool grid_sums(const double (&v)[NV], double* partials, unsigned* ticket,
                                           int nblocks, double (&out)[NV], int bid = -1) {
-    __shared__ double red[NT / 32];
+    // The values go through the same two steps together: the tail of a reduction is a chain of latencies (block
+    // sum, arrival, the last block's loads and its sum), 4 us of a 9 us kernel on 64^3 cells when they
+    // went one after the other through one thread's additions.
+    constexpr int NW = NT / 32;
+    __shared__ double red[NV][NW];
     __shared__ bool s_last;
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
     if (bid < 0) bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    for (int q = 0; q < NV; ++q) {
-        double s = block_sum<NT>(v[q], red);
-        if (tid == 0) partials[(size_t)q * nblocks + bid] = s;
-    }
+    // sums of every thread's v over the block, on thread 0
+    auto block_sums = [&](double (&x)[NV]) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) x[q] += __shfl_down_sync(0xffffffffu, x[q], o);
+        if ((tid & 31) == 0)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) red[q][tid >> 5] = x[q];
+        __syncthreads();
+        if (tid < 32) {
+#pragma unroll
+            for (int q = 0; q < NV; ++q) x[q] = tid < NW ? red[q][tid] : 0.0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                if (o < NW)
+#pragma unroll
+                    for (int q = 0; q < NV; ++q) x[q] += __shfl_down_sync(0xffffffffu, x[q], o);
+        }
+    };
+    double x[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) x[q] = v[q];
+    block_sums(x);
     if (tid == 0) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) partials[(size_t)q * nblocks + bid] = x[q];
         __threadfence();
-        unsigned t = atomicAdd(ticket, 1u);
+        const unsigned t = atomicAdd(ticket, 1u);
         s_last = (t == (unsigned)nblocks - 1);
     }
     __syncthreads();
     if (!s_last) return false;
     __threadfence();
-    for (int q = 0; q < NV; ++q) {
-        double acc = 0.0;
-        for (int b = tid; b < nblocks; b += NT) acc += __ldcg(partials + (size_t)q * nblocks + b);
-        out[q] = block_sum<NT>(acc, red);
+#pragma unroll
+    for (int q = 0; q < NV; ++q) x[q] = 0.0;
+#pragma unroll 4
+    for (int b = tid; b < nblocks; b += NT)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) x[q] += __ldcg(partials + (size_t)q * nblocks + b);
+    __syncthreads(); // (red of the first step has been read)
+    block_sums(x);
+    if (tid == 0) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) out[q] = x[q];
+        *ticket = 0u;
     }
-    if (tid == 0) *ticket = 0u;
     return tid == 0;
 }
 

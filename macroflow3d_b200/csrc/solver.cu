@@ -104,6 +104,14 @@ static ColLaunch col_launch(int nx, int ny, int nz, int per_sm = 8) {
     return L;
 }
 
+// ... of the kernels that stage planes around a chunk (matvec: two more than it applies): chunks of at least
+// four planes as long as every SM has a block
+static ColLaunch col_launch_staged(int nx, int ny, int nz, int per_sm) {
+    const long long tiles = (long long)((nx + 31) / 32) * ((ny + 7) / 8);
+    while (per_sm > 1 && tiles * ((nz + 3) / 4) < (long long)num_sms() * per_sm) --per_sm;
+    return col_launch(nx, ny, nz, per_sm);
+}
+
 // RAII device allocation
 struct DevMem {
     void* p = nullptr;
@@ -722,6 +730,12 @@ template <class T, class TC> class VCycle : public VCycleBase {
             }
             if (n_pair_) set_pair_smem();
         }
+        // levels whose legs run in bricks (kernels_brick.cuh): two sweeps a leg, and few enough bricks
+        brick_.assign(Lt, 0);
+        for (int l = 0; l < Lt; ++l) {
+            const dim3 g = brick_grid(G[l]);
+            brick_[l] = pre == 2 && post == 2 && (long long)g.x * g.y * g.z <= (long long)kBrickWaves * num_sms();
+        }
         // coarse tail: FP64 weights per cell, x (ghost-padded) and b in shared memory
         if (Lt < nl) {
             tail_.nlev = nl - Lt;
@@ -730,12 +744,6 @@ template <class T, class TC> class VCycle : public VCycleBase {
             tail_.post = post;
             tail_.coarse_iters = coarse;
             // weights of every level either coarse kernel serves: [Lw, coarsest)
-        // levels whose legs run in bricks (kernels_brick.cuh): two sweeps a leg, and few enough bricks
-        brick_.assign(Lt, 0);
-        for (int l = 0; l < Lt; ++l) {
-            const dim3 g = brick_grid(G[l]);
-            brick_[l] = pre == 2 && post == 2 && (long long)g.x * g.y * g.z <= (long long)kBrickWaves * num_sms();
-        }
             Lw_ = cp_.Lc >= 0 ? std::min(cp_.Lc, Lt) : Lt;
             size_t wtot = 0;
             for (int l = Lw_; l < nl; ++l) wtot += 8 * G[l].n;
@@ -783,6 +791,7 @@ template <class T, class TC> class VCycle : public VCycleBase {
                 T2.w = tail_w_->as<double>() + woff;
                 woff += 8 * G[l].n;
             }
+            plan_dense(nl);
             tail_smem_ = (size_t)off * sizeof(double);
             tail_out_.reset(new DevMem(G[Lt].n * sizeof(T)));
             bytes_ += G[Lt].n * sizeof(T);
@@ -791,7 +800,6 @@ template <class T, class TC> class VCycle : public VCycleBase {
             // not lower it under this one
             if (tail_smem_ > kTailSmemMax) throw Error(MF3D_E_INVALID, "coarse tail exceeds shared memory");
             MF3D_CK(cudaFuncSetAttribute(tail2_kernel<T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            plan_dense(nl);
                                          (int)kTailSmemMax));
             MF3D_CK(cudaFuncSetAttribute(tail2_kernel<double, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kTailSmemMax));
@@ -864,6 +872,11 @@ template <class T, class TC> class VCycle : public VCycleBase {
         for (int l = 0; l < Lb; ++l) {
             T* bc_next = (T*)bl_[l + 1]->p;
             const T* c = nullptr;
+            if (brick_[l] && !rec_) {
+                brick_leg(s, l, nullptr, (T*)xa_[l]->p, nullptr, bc_next, nullptr);
+                cur[l] = (const T*)xa_[l]->p;
+                continue;
+            }
             for (int sw = 1; sw <= pre_; ++sw) {
                 T* out = other(l, c);
                 int mode = (c ? 0 : M_ZERO) | (sw == pre_ ? M_RESID : 0);
@@ -872,11 +885,6 @@ template <class T, class TC> class VCycle : public VCycleBase {
                 // staged levels: the last pre-sweep, then the residual and its restriction in a
                 // kernel of their own (batched solves record the fused form)
                 const bool split = (mode & M_RESID) && (tma_[l] || pair_[l]) && split_resid_ && !rec_;
-            if (brick_[l] && !rec_) {
-                brick_leg(s, l, nullptr, (T*)xa_[l]->p, nullptr, bc_next, nullptr);
-                cur[l] = (const T*)xa_[l]->p;
-                continue;
-            }
                 sweep(s, l, c, out, nullptr, split ? nullptr : bc_next, split ? (mode & ~M_RESID) : mode, nullptr);
                 if (split) resid_restrict(s, l, out, bc_next);
                 c = out;
@@ -896,6 +904,12 @@ template <class T, class TC> class VCycle : public VCycleBase {
         for (int l = Lb - 1; l >= 0; --l) {
             const T* c = cur[l];
             const T* e = (l + 1 == Lb) ? e_below : fin[l + 1];
+            if (brick_[l] && !rec_) {
+                T* out = l == 0 ? z : other(l, c);
+                brick_leg(s, l, c, out, e, nullptr, l == 0 ? rho_out : nullptr);
+                fin[l] = out;
+                continue;
+            }
             for (int sw = 1; sw <= post_; ++sw) {
                 const bool last = sw == post_;
                 T* out = (l == 0 && last) ? z : other(l, c);
@@ -904,12 +918,6 @@ template <class T, class TC> class VCycle : public VCycleBase {
                 rec_sw_ = 2 * sw; // (2 sw + 1: the residual + restriction after it)
                 sweep(s, l, c, out, e, nullptr, mode, rho_out);
                 c = out;
-            if (brick_[l] && !rec_) {
-                T* out = l == 0 ? z : other(l, c);
-                brick_leg(s, l, c, out, e, nullptr, l == 0 ? rho_out : nullptr);
-                fin[l] = out;
-                continue;
-            }
             }
             if (post_ == 0) {
                 T* out = (l == 0) ? z : other(l, c);
@@ -989,6 +997,7 @@ template <class T, class TC> class VCycle : public VCycleBase {
                 }), et * n + et * n + coef + et * n + 8.0 * n + (post_ == 1 ? et * nc : 0.0), 1));
             }
             for (int l = 1; l < Lb; ++l) {
+                if (brick_[l]) continue;
                 std::snprintf(nm, sizeof(nm), "sweep_l%d_plain_%s", l, pair_[l] ? "pair" : (tma_[l] ? "tma" : "ldg"));
                 T* a = (T*)xa_[l]->p;
                 T* b = (T*)xb_[l]->p;
@@ -997,7 +1006,6 @@ template <class T, class TC> class VCycle : public VCycleBase {
                                      3.0 * et * nn + 3.0 * nn * ec, pre_ + post_));
             }
         }
-                if (brick_[l]) continue;
         if (Lb < nl) {
             T* outp = coarse_out(z);
             out.push_back(timing(dense_on() ? "coarse_bricks_matrix" : cluster_on() ? "coarse_cluster" : "coarse_tail",
@@ -1012,14 +1020,6 @@ template <class T, class TC> class VCycle : public VCycleBase {
 
     T* other(int l, const T* c) const { return (c == (const T*)xa_[l]->p) ? (T*)xb_[l]->p : (T*)xa_[l]->p; }
 
-    // the cluster kernel serves this solve's coarse end (single solves with a plan)
-    bool cluster_on() const { return cp_.Lc >= 0 && !rec_tail_ && !rec_; }
-    int coarse_start() const { return cluster_on() ? cp_.Lc : Lt_; }
-    // where the coarse end writes its correction: z when it is the whole V-cycle
-    T* coarse_out(T* z) const {
-        const int Lb = coarse_start();
-        if (Lb == 0) return z;
-        if (cluster_on() && Lb < Lt_) return (T*)ctail_out_->p;
     // Bricks of a level whose legs run in one launch each: up to kBrickWaves per SM.  A wave
     // takes about 6.5 us a leg whatever the level, the five launches it replaces about 30 us on 32^3 to 64^3 cells
     // (FP32: 48^3, 216 bricks, 31.5 us in bricks and 31 us as sweeps; 64^3, 512 bricks, 59 and 40 us; FP64:
@@ -1051,9 +1051,9 @@ template <class T, class TC> class VCycle : public VCycleBase {
         MF3D_LAUNCH_CK();
     }
 
-        return (T*)tail_out_->p;
-    }
-
+    // the cluster kernel serves this solve's coarse end (single solves with a plan)
+    bool cluster_on() const { return cp_.Lc >= 0 && !rec_tail_ && !rec_; }
+    int coarse_start() const { return cluster_on() ? cp_.Lc : Lt_; }
     // ---- the FP64 levels of a single solve as bricks and one matrix ----
     // The levels from the first FP64 one down to D_ (the first of at most DN_MAX cells, or the coarsest one of
     // at most DN_MAX_LAST) run their legs in bricks, and the cycle from D_ on is a matrix product.  Where
@@ -1137,7 +1137,20 @@ template <class T, class TC> class VCycle : public VCycleBase {
         }
     }
 
+    // where the coarse end writes its correction: z when it is the whole V-cycle
+    T* coarse_out(T* z) const {
+        const int Lb = coarse_start();
+        if (Lb == 0) return z;
+        if (cluster_on() && Lb < Lt_) return (T*)ctail_out_->p;
+        return (T*)tail_out_->p;
+    }
+
     void launch_tail(cudaStream_t s, T* out) {
+        if (dense_on()) {
+            if (coarse_start() == 0) dense_end(s, r64_, out);
+            else dense_end(s, (const T*)bl_[coarse_start()]->p, out);
+            return;
+        }
         if (cluster_on()) {
             if (cp_.Lc == 0)
                 launch_coarse<double, T>(s, cp_, cp_.a, r64_, out);
@@ -1146,11 +1159,6 @@ template <class T, class TC> class VCycle : public VCycleBase {
             return;
         }
         if (rec_tail_) { // batched solve: record only (the batch needs a level above the tail)
-        if (dense_on()) {
-            if (coarse_start() == 0) dense_end(s, r64_, out);
-            else dense_end(s, (const T*)bl_[coarse_start()]->p, out);
-            return;
-        }
             if (Lt_ == 0) throw Error(MF3D_E_INVALID, "batched solve: the whole hierarchy fits the coarse tail");
             rec_tail_->a = tail_;
             rec_tail_->b = (const T*)bl_[Lt_]->p;
@@ -1472,21 +1480,13 @@ template <class T, class TC> class VCycle : public VCycleBase {
     // 0.152 + 0.069 ms against 0.280 ms).  Batched solves keep the fused sweep.
     static constexpr bool split_resid_ = sizeof(TC) >= 4 || kPair;
     int occ_[16] = {}; // resident staged-sweep CTAs per SM, by mode
+    std::vector<int> brick_;   // levels whose legs run in bricks
     std::vector<int> pair_;    // levels served by the x-pair sweep
     std::vector<int> pair_tm_; // ... with TMA staging
     std::vector<std::array<SpMaps, 2>> pmaps_; // their tensor maps, x read from xa / xb
     int n_pair_ = 0;
     int pocc_[16] = {}, pocc_tm_[16] = {}; // resident x-pair-sweep CTAs per SM, by mode
     std::unique_ptr<DevMem> tail_out_, tail_w_, ctail_out_, cmap_;
-    Tail2Args tail_{};
-    int Lw_ = 0; // first level with FP64 weights
-    std::vector<int> brick_;   // levels whose legs run in bricks
-    size_t tail_smem_ = 0;
-    size_t bytes_ = 0;
-};
-
-template <class T>
-__global__ void dot_kernel(size_t n, const double* __restrict__ a, const T* __restrict__ b, double* partials,
     struct Coarse64 {
         double *b = nullptr, *x = nullptr, *y = nullptr;
     };
@@ -1495,6 +1495,14 @@ __global__ void dot_kernel(size_t n, const double* __restrict__ a, const T* __re
     Tail2Args dtail_{};
     int D_ = 0, dense_ld_ = 0;
     size_t dtail_smem_ = 0;
+    Tail2Args tail_{};
+    int Lw_ = 0; // first level with FP64 weights
+    size_t tail_smem_ = 0;
+    size_t bytes_ = 0;
+};
+
+template <class T>
+__global__ void dot_kernel(size_t n, const double* __restrict__ a, const T* __restrict__ b, double* partials,
                            unsigned* ticket, double* out) {
     double acc = 0.0;
     for (size_t c = blockIdx.x * (size_t)PK_NT + threadIdx.x; c < n; c += (size_t)gridDim.x * PK_NT)
@@ -1511,12 +1519,14 @@ void VCycle<T, TC>::dot_rz(cudaStream_t s, const T* z, size_t n, double* out) {
 }
 
 template <class T, class TC> class BatchSolverT;
+class EnsembleSolver;
 
 // ---------------------------------------------------------------------------------------
 // HeadSolver
 // ---------------------------------------------------------------------------------------
 class HeadSolver {
     template <class T, class TC> friend class BatchSolverT;
+    friend class EnsembleSolver;
 
   public:
     HeadSolver(const mf3d_grid& g, const mf3d_bc& bc, const mf3d_solver_config& cfg, cudaStream_t user_stream)
@@ -1655,14 +1665,6 @@ class HeadSolver {
     void set_K(const double* K, cudaStream_t s) {
         if (!K) throw Error(MF3D_E_INVALID, "K is null");
         const long long l0 = g_launches;
-        enqueue(h, x0, stream_);
-        MF3D_CK(cudaStreamSynchronize(stream_));
-        finish(res);
-    }
-
-    // The whole solve on stream s, its state copied to the host at the end; with use_graph nothing here
-    // waits.  finish() after the stream has been waited for.
-    void enqueue(double* h, const double* x0, cudaStream_t s) {
         const int nl = (int)G_.size();
         MF3D_CK(cudaMemcpyAsync(Klev_[0]->p, K, G_[0].n * sizeof(double), cudaMemcpyDeviceToDevice, s));
         for (int l = 0; l + 1 < nl; ++l) {
@@ -1682,14 +1684,12 @@ class HeadSolver {
             rhs_guess_kernel<<<cl.grid, cl.block, 0, s>>>(G_[0].nx, G_[0].ny, G_[0].nz, G_[0].dx, Kp[0], to_dev(bc_),
                                                           b_.as<double>(), x0_.as<double>(), cl.zchunk);
         }
-class EnsembleSolver;
         MF3D_LAUNCH_CK();
         setup_launches_ = (int)(g_launches - l0);
         have_K_ = true;
     }
 
     int setup_launches() const { return setup_launches_; }
-    friend class EnsembleSolver;
     void set_budget_ns(unsigned long long ns) { budget_ns_ = ns; }
 
     void vcycle(const double* r, double* z) {
@@ -1723,6 +1723,14 @@ class EnsembleSolver;
     void solve(double* h, const double* x0, mf3d_solve_result* res) {
         if (!have_K_) throw Error(MF3D_E_STATE, "set_K must be called before solve");
         if (!h) throw Error(MF3D_E_INVALID, "h is null");
+        enqueue(h, x0, stream_);
+        MF3D_CK(cudaStreamSynchronize(stream_));
+        finish(res);
+    }
+
+    // The whole solve on stream s, its state copied to the host at the end; with use_graph nothing here
+    // waits.  finish() after the stream has been waited for.
+    void enqueue(double* h, const double* x0, cudaStream_t s) {
         const size_t n = G_[0].n;
         const long long l0 = g_launches;
         body_runs_ = 0;
@@ -1749,6 +1757,11 @@ class EnsembleSolver;
                 MF3D_CK(cudaStreamSynchronize(s));
                 if (host_state_->stop) break;
             }
+        }
+        if (!mg) {
+            xfinish_kernel<<<grid1d(n, PK_NT), PK_NT, 0, s>>>(n, x_.as<double>(), p_.as<double>(), p2_.as<double>(),
+                                                              state_.as<PcgState>());
+            MF3D_LAUNCH_CK();
         }
         launch_residual(s, 1);
         MF3D_CK(cudaMemcpyAsync(h, x_.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
@@ -1798,17 +1811,15 @@ class EnsembleSolver;
         out.push_back(timing("residual_true", tm.mean_ms(reps, [&] { launch_residual(stream_, 1); }), 48.0 * nd, 0));
         out.push_back(timing("xr_update", tm.mean_ms(reps, [&] {
             if (vc_->z_elt() == sizeof(double))
-                xr_update_kernel<double><<<nb, PK_NT, 0, stream_>>>(n, x_.as<double>(), p_.as<double>(), r_.as<double>(),
-                                                                   Ap_.as<double>(), z_.as<double>(), st,
+                xr_update_kernel<double><<<nb, PK_NT, 0, stream_>>>(n, r_.as<double>(), Ap_.as<double>(), z_.as<double>(), st,
                                                                    partials_.as<double>(), tickets_.as<unsigned>() + 4,
-                                                                   cond_, 0, r32_.as<float>(), p2_.as<double>());
+                                                                   cond_, 0, r32_.as<float>());
             else
-                xr_update_kernel<float><<<nb, PK_NT, 0, stream_>>>(n, x_.as<double>(), p_.as<double>(), r_.as<double>(),
-                                                                  Ap_.as<double>(), z_.as<float>(), st,
+                xr_update_kernel<float><<<nb, PK_NT, 0, stream_>>>(n, r_.as<double>(), Ap_.as<double>(), z_.as<float>(), st,
                                                                   partials_.as<double>(), tickets_.as<unsigned>() + 4,
-                                                                  cond_, 0, r32_.as<float>(), p2_.as<double>());
+                                                                  cond_, 0, r32_.as<float>());
             MF3D_LAUNCH_CK();
-        }), 48.0 * nd + (flexible_ ? ez * nd : 0.0), 1));
+        }), 24.0 * nd + (flexible_ ? ez * nd : 0.0) + (r32_.p ? 4.0 * nd : 0.0), 1));
         return out;
     }
 
@@ -1819,7 +1830,7 @@ class EnsembleSolver;
     // p = z + beta p fused with Ap = A p and <p, Ap> (z = r for plain CG)
     void launch_pmatvec(cudaStream_t s) {
         PcgState* st = state_.as<PcgState>();
-        const ColLaunch cl = col_launch(G_[0].nx, G_[0].ny, G_[0].nz, MF3D_PMATVEC_PERSM);
+        const ColLaunch cl = col_launch_staged(G_[0].nx, G_[0].ny, G_[0].nz, MF3D_PMATVEC_PERSM);
         const bool z64 = cfg_.solver == MF3D_SOLVER_CG || vc_->z_elt() == sizeof(double);
         // per call: the attribute belongs to the current device
         if (z64)
@@ -1831,11 +1842,11 @@ class EnsembleSolver;
         if (z64) {
             const double* z = cfg_.solver == MF3D_SOLVER_CG ? r_.as<double>() : z_.as<double>();
             pmatvec_dot_kernel<double><<<cl.grid, cl.block, pmv_smem_bytes<double>(), s>>>(
-                op64_[0], z, p_.as<double>(), p2_.as<double>(), Ap_.as<double>(), st, partials_.as<double>(),
+                op64_[0], z, p_.as<double>(), p2_.as<double>(), Ap_.as<double>(), x_.as<double>(), st, partials_.as<double>(),
                 tickets_.as<unsigned>() + 3, cl.zchunk);
         } else {
             pmatvec_dot_kernel<float><<<cl.grid, cl.block, pmv_smem_bytes<float>(), s>>>(
-                op64_[0], z_.as<float>(), p_.as<double>(), p2_.as<double>(), Ap_.as<double>(), st,
+                op64_[0], z_.as<float>(), p_.as<double>(), p2_.as<double>(), Ap_.as<double>(), x_.as<double>(), st,
                 partials_.as<double>(), tickets_.as<unsigned>() + 3, cl.zchunk);
         }
         MF3D_LAUNCH_CK();
@@ -1879,15 +1890,13 @@ class EnsembleSolver;
         launch_pmatvec(s);
         if (cg || z64) {
             const double* z = cg ? r_.as<double>() : z_.as<double>();
-            xr_update_kernel<double><<<nb, PK_NT, 0, s>>>(n, x_.as<double>(), p_.as<double>(), r_.as<double>(),
-                                                          Ap_.as<double>(), z, st, partials_.as<double>(),
+            xr_update_kernel<double><<<nb, PK_NT, 0, s>>>(n, r_.as<double>(), Ap_.as<double>(), z, st, partials_.as<double>(),
                                                           tickets_.as<unsigned>() + 4, cond_, with_cond ? 1 : 0,
-                                                          r32_.as<float>(), p2_.as<double>());
+                                                          r32_.as<float>());
         } else {
-            xr_update_kernel<float><<<nb, PK_NT, 0, s>>>(n, x_.as<double>(), p_.as<double>(), r_.as<double>(),
-                                                         Ap_.as<double>(), z_.as<float>(), st, partials_.as<double>(),
+            xr_update_kernel<float><<<nb, PK_NT, 0, s>>>(n, r_.as<double>(), Ap_.as<double>(), z_.as<float>(), st, partials_.as<double>(),
                                                          tickets_.as<unsigned>() + 4, cond_, with_cond ? 1 : 0,
-                                                         r32_.as<float>(), p2_.as<double>());
+                                                         r32_.as<float>());
         }
         MF3D_LAUNCH_CK();
     }
