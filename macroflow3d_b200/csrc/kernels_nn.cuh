@@ -7,18 +7,11 @@
 // v * C + c, v = i + nx (j + ny k).  Weights of a 3x3x3 convolution are [cout][27][cin] with
 // tap t = (dz+1)*9 + (dy+1)*3 + (dx+1).
 //
-// conv3d_tc_kernel: implicit GEMM on the 5th-generation tensor cores.  D[v][co] =
-// sum_{t, ci} X[v + off(t)][ci] W[co][t][ci]: M = 128 voxels per tile, N = cout, K = 27 cin
-// in steps of 16 channels.  Per tap, the CTA gathers the 128 x cin activation tile (zero
-// outside the grid) and the cout x cin weight tile into shared memory in the canonical
-// K-major, non-swizzled UMMA layout (8-row x 16-byte core matrices; the two 8-channel halves
-// of a 16-channel step 128 bytes apart, 8-row groups 256 bytes apart), one thread issues the
-// cin/16 tcgen05.mma of the tap into a TMEM accumulator (128 lanes x cout FP32 columns) and
-// commits them to the tap's mbarrier, and the CTA gathers the next tap into the other buffer
-// meanwhile.  The epilogue reads TMEM with tcgen05.ld (warp w owns lanes 32w..32w+31), adds
-// the bias, applies ReLU or a ReLU-derivative mask, and stores BF16 or FP32.  The data
-// gradient of a convolution is the same kernel on the output gradient with the weights
-// flipped in the taps and transposed in the channels.
+// conv3d_brick_kernel: implicit GEMM on the 5th-generation tensor cores.  D[v][co] =
+// sum_{t, ci} X[v + off(t)][ci] W[co][t][ci]: M = 128 voxels, N = output channels of three output planes,
+// K = 27 cin in steps of 16 channels, FP32 accumulators in TMEM.  The data gradient of a convolution is
+// the same kernel on the output gradient with the weights flipped in the taps and transposed in the
+// channels.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -29,7 +22,6 @@
 namespace mf3d {
 namespace nn {
 
-constexpr int CONV_NT = 128;   // 4 warps: one TMEM lane quarter each
 constexpr int CONV_TM = 128;   // voxels per tile (UMMA M)
 constexpr int CONV_MAXC = 128; // channel limit (multiples of 16)
 
@@ -53,22 +45,14 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// D(tmem) (+)= A(smem desc) * B(smem desc)^T, kind::f16 (BF16 inputs, FP32 accumulate)
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
-                 "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-                 : "memory");
-}
 // One lane of the warp, the same one for the same (full) mask.
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t r;
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
     return r;
 }
-// The same product, called by a whole warp in uniform control flow and issued by its elected lane:
-// the descriptors then stay in uniform registers.  From one lane's own branch every product
+// D(tmem) (+)= A(smem desc) * B(smem desc)^T, kind::f16 (BF16 inputs, FP32 accumulate), called by a whole warp in
+// uniform control flow and issued by its elected lane: the descriptors then stay in uniform registers.  From one lane's own branch every product
 // moved its descriptors there first, which took longer than the product (16 -> 16 channels at 128^3:
 // 127 cycles a product).  Descriptors as (low, high) words; only the low one carries the start address.
 __device__ __forceinline__ void umma_bf16_warp(uint32_t d_tmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
@@ -86,10 +70,6 @@ __device__ __forceinline__ void umma_commit_warp(uint64_t* bar, uint32_t leader)
                  "r"(leader)
                  : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sm_u32(bar))
-                 : "memory");
-}
 // 16 consecutive FP32 columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
@@ -103,6 +83,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
+
+// 16 columns of this thread's TMEM lane = 0; complete after tmem_wait_st
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+                 "r"(0u)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void nn_mbar_init(uint64_t* bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sm_u32(bar)), "r"(count) : "memory");
@@ -122,22 +110,10 @@ __device__ __forceinline__ bool nn_mbar_wait(uint64_t* bar, unsigned parity, int
     return false;
 }
 
-// Shared-memory matrix descriptor of a K-major, non-swizzled operand tile: start address,
-// leading byte offset (between the two 8-element K halves) 128 B, stride byte offset (between
-// 8-row groups) 256 B, descriptor version 1 (sm_100), layout type 0 (no swizzle).
-__device__ __forceinline__ uint64_t kmajor_desc(uint32_t saddr) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(256u >> 4) << 32) |
-           (1ull << 46);
-}
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both K-major, M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-// byte offset of (row, k) in a K-major tile of `rows` rows and 16 K-columns
-__device__ __forceinline__ uint32_t kmajor_off(int row, int khalf) {
-    return (uint32_t)((row >> 3) * 256 + khalf * 128 + (row & 7) * 16);
-}
-
 struct ConvArgs {
     const __nv_bfloat16* x; // [V][cin]
     const __nv_bfloat16* w; // [cout][27][cin]
@@ -149,179 +125,27 @@ struct ConvArgs {
     int* err; // set when an mbarrier wait gives up
 };
 
-// shared memory of conv3d_tc_kernel for (cin, cout): two buffers of (A 128 x cin, B cout x cin)
-__host__ __device__ constexpr size_t conv_smem(int cin, int cout) {
-    return 2 * ((size_t)CONV_TM * cin * 2 + (size_t)cout * cin * 2) + 64;
-}
 __host__ __device__ constexpr uint32_t tmem_cols(int cout) {
     return cout <= 32 ? 32u : cout <= 64 ? 64u : cout <= 128 ? 128u : cout <= 256 ? 256u : 512u;
 }
 
-__global__ void __launch_bounds__(CONV_NT) conv3d_tc_kernel(const ConvArgs a) {
-    extern __shared__ __align__(1024) unsigned char nn_sm[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int cin = a.cin, cout = a.cout;
-    const size_t abytes = (size_t)CONV_TM * cin * 2, bbytes = (size_t)cout * cin * 2;
-    unsigned char* buf[2] = {nn_sm, nn_sm + abytes + bbytes};
-    uint64_t* bars = reinterpret_cast<uint64_t*>(nn_sm + 2 * (abytes + bbytes)); // 2 mbarriers
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
-    const uint32_t ncols = tmem_cols(cout);
-    if (warp == 0) {
-        tmem_alloc(tmem_slot, ncols);
-        tmem_relinquish();
-    }
-    if (tid == 0) {
-        nn_mbar_init(&bars[0], 1);
-        nn_mbar_init(&bars[1], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const int nx = a.nx, ny = a.ny, nz = a.nz;
-    const long long V = (long long)nx * ny * nz;
-    const int ntiles = (int)((V + CONV_TM - 1) / CONV_TM);
-    const uint32_t idesc = idesc_bf16(CONV_TM, cout);
-    const int ksteps = cin / 16;
-    unsigned phase[2] = {0u, 0u};
-    int pending[2] = {0, 0}; // commits issued and not yet waited for, per buffer
-    bool fail = false;
-
-    for (int tile = blockIdx.x; tile < ntiles && !fail; tile += gridDim.x) {
-        const long long v = (long long)tile * CONV_TM + tid; // this thread's row
-        const bool vin = v < V;
-        int vi = 0, vj = 0, vk = 0;
-        if (vin) {
-            vi = (int)(v % nx);
-            vj = (int)((v / nx) % ny);
-            vk = (int)(v / ((long long)nx * ny));
-        }
-        for (int t = 0; t < 27 && !fail; ++t) {
-            const int b = t & 1;
-            // the buffer's previous MMAs must have finished reading it
-            if (pending[b]) {
-                if (!nn_mbar_wait(&bars[b], phase[b])) fail = true;
-                phase[b] ^= 1u;
-                pending[b] = 0;
-            }
-            if (__syncthreads_or(fail)) {
-                fail = true;
-                break;
-            }
-            const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dxo = t % 3 - 1;
-            // ---- A: this thread's voxel row, cin channels of its neighbour at tap t ----
-            {
-                const int ii = vi + dxo, jj = vj + dy, kk = vk + dz;
-                const bool ok = vin && ii >= 0 && ii < nx && jj >= 0 && jj < ny && kk >= 0 && kk < nz;
-                const uint4* src = ok ? reinterpret_cast<const uint4*>(a.x + ((size_t)ii + (size_t)nx * ((size_t)jj + (size_t)ny * kk)) * cin)
-                                      : nullptr;
-                unsigned char* A = buf[b];
-                for (int c = 0; c < cin / 8; ++c) {
-                    const uint4 val = ok ? __ldg(src + c) : make_uint4(0u, 0u, 0u, 0u);
-                    *reinterpret_cast<uint4*>(A + (size_t)(c >> 1) * (CONV_TM * 32) + kmajor_off(tid, c & 1)) = val;
-                }
-            }
-            // ---- B: the weights of tap t ----
-            {
-                unsigned char* B = buf[b] + abytes;
-                const int chunks = cout * (cin / 8);
-                for (int q = tid; q < chunks; q += CONV_NT) {
-                    const int n = q / (cin / 8), c = q % (cin / 8);
-                    const uint4 val = __ldg(reinterpret_cast<const uint4*>(a.w + ((size_t)n * 27 + t) * cin) + c);
-                    *reinterpret_cast<uint4*>(B + (size_t)(c >> 1) * (cout * 32) + kmajor_off(n, c & 1)) = val;
-                }
-            }
-            // generic-proxy writes to shared memory, then visible to the tensor core
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncthreads();
-            if (tid == 0) {
-                tc_fence_after();
-                const uint32_t abase = sm_u32(buf[b]), bbase = sm_u32(buf[b] + abytes);
-                for (int s = 0; s < ksteps; ++s)
-                    umma_bf16(tmem, kmajor_desc(abase + s * (CONV_TM * 32)), kmajor_desc(bbase + s * (cout * 32)),
-                              idesc, (t > 0 || s > 0) ? 1u : 0u);
-                umma_commit(&bars[b]);
-            }
-            pending[b] = 1;
-        }
-        // ---- epilogue: wait for the last MMAs, then TMEM -> registers -> global ----
-        for (int b = 0; b < 2; ++b)
-            if (pending[b]) {
-                if (!nn_mbar_wait(&bars[b], phase[b])) fail = true;
-                phase[b] ^= 1u;
-                pending[b] = 0;
-            }
-        fail = __syncthreads_or(fail);
-        if (fail) break;
-        tc_fence_after();
-        const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int c0 = 0; c0 < cout; c0 += 16) {
-            float acc[16];
-            tmem_ld16(lane_base + (uint32_t)c0, acc);
-            if (vin) {
-                if (a.bias)
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) acc[i] += __ldg(a.bias + c0 + i);
-                if (a.relu)
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) acc[i] = fmaxf(acc[i], 0.f);
-                if (a.mask) {
-                    const uint4* mp = reinterpret_cast<const uint4*>(a.mask + (size_t)v * cout + c0);
-                    const uint4 m0 = __ldg(mp), m1 = __ldg(mp + 1);
-                    const __nv_bfloat16* mb0 = reinterpret_cast<const __nv_bfloat16*>(&m0);
-                    const __nv_bfloat16* mb1 = reinterpret_cast<const __nv_bfloat16*>(&m1);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        if (!(__bfloat162float(mb0[i]) > 0.f)) acc[i] = 0.f;
-                        if (!(__bfloat162float(mb1[i]) > 0.f)) acc[8 + i] = 0.f;
-                    }
-                }
-                if (a.y_f32) {
-                    float4* yp = reinterpret_cast<float4*>(static_cast<float*>(a.y) + (size_t)v * cout + c0);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) yp[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
-                } else {
-                    __align__(16) __nv_bfloat16 o[16];
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) o[i] = __float2bfloat16(acc[i]);
-                    uint4* yp = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.y) + (size_t)v * cout + c0);
-                    yp[0] = reinterpret_cast<const uint4*>(o)[0];
-                    yp[1] = reinterpret_cast<const uint4*>(o)[1];
-                }
-            }
-        }
-        // every warp has read its lanes before the next tile's MMAs overwrite them
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-    }
-    if (fail) {
-        if (tid == 0) atomicExch(a.err, 1);
-        // wait (bounded) for MMAs still in flight before the accumulator is released
-        for (int b = 0; b < 2; ++b)
-            if (pending[b]) (void)nn_mbar_wait(&bars[b], phase[b]);
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        tc_fence_after();
-        tmem_dealloc(tmem, ncols);
-    }
-}
-
-// ---- conv3d_brick_kernel: the same convolution with the halo staged once per plane ----
-// A CTA owns a 16 x 16 voxel brick (two 8 x 16 UMMA M-tiles) and marches it through a z
-// range.  Producer warps stage each input plane of the brick plus a one-voxel halo
-// (18 x 18 voxels x cin) into a ring of 4 plane slots with cp.async (zero fill outside the
-// grid), one region per 8-channel half so that every tap's A operand is the same K-major
-// canonical layout at a shifted start address: rows of 8 voxels along x at 16 bytes, 8-row
-// groups (y) 18 x 16 = 288 bytes apart, the two channel halves of a 16-channel K-step one
-// region (18 x 18 x 16 = 5184 bytes) apart.  The weights of all 27 taps stay in shared memory.
-// One thread issues the 27 x cin/16 x 2 MMAs of an output plane into one of two TMEM
-// accumulator buffers and commits them; four epilogue warps drain the other buffer
-// meanwhile (bias, ReLU or mask, BF16 / FP32 store).  Every wait is bounded.
+// ---- conv3d_brick_kernel ----
+// A CTA owns a brick of A UMMA M-tiles (8 x 16 voxels each, side by side in x) and marches it through a z
+// range.  Producer warps stage each input plane of the brick plus a one-voxel halo into a ring of plane
+// slots with cp.async (zero fill outside the grid), one region per 8-channel group so that every (dy, dx)
+// tap's A operand is the same K-major canonical layout at a shifted start address: rows of 8 voxels along
+// x at 16 bytes, 8-row groups (y) a halo row apart, the two channel halves of a 16-channel K step one
+// region apart.  The weights of all 27 taps stay in shared memory.
+// A plane p is read once: it contributes to the output planes p-1, p and p+1, whose accumulators lie side
+// by side in TMEM (a ring of four planes), so one product per (dy, dx), K step and tile has N = 3 coutp columns,
+// the weights of dz = +1, 0, -1 (two products where the ring wraps).  A product reads a 4 KB A tile whatever
+// N is and takes about 70 cycles with 16 columns, 100 with 48.  One warp issues them; four epilogue
+// warps drain an output plane that is complete (bias, ReLU or mask, BF16 / FP32 store) and clear it for the
+// plane that takes its place, while the products of the next plane run.  Every wait is bounded.
+// 16 -> 16 channels at 128^3: 0.145 ms with one product per tap and plane -> 0.101 ms; 48 -> 16: 0.442 -> 0.259 ms;
+// 128 -> 64 at 32^3: 0.310 ms when its taps were gathered into shared memory -> 0.111 ms in four launches.
 constexpr int BR_MAXNP = 8;                    // input plane slots, at most
+constexpr int BR_OUT = 4;                      // output planes in TMEM: three in work, one being drained
 constexpr int BR_PROD = 4, BR_EPI = 4;         // producer and epilogue warps
 constexpr int BR_NT = (BR_PROD + 1 + BR_EPI) * 32;
 // Brick geometry: A UMMA M-tiles of 8 x 16 voxels side by side in x (brick 8A x 16), a ring of
@@ -331,7 +155,7 @@ __host__ __device__ constexpr size_t brick_slot_bytes(int A, int cin) { return (
 __host__ __device__ constexpr size_t brick_smem(int A, int NP, int cin, int coutp) {
     return (size_t)27 * coutp * cin * 2 + NP * brick_slot_bytes(A, cin) + 256;
 }
-__host__ __device__ constexpr uint32_t brick_tmem_cols(int A, int coutp) { return tmem_cols(2 * A * coutp); }
+__host__ __device__ constexpr uint32_t brick_tmem_cols(int A, int coutp) { return tmem_cols(BR_OUT * A * coutp); }
 
 // K-major descriptor with explicit leading / stride byte offsets
 __device__ __forceinline__ uint64_t kdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
@@ -367,19 +191,19 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
     uint64_t* bars = reinterpret_cast<uint64_t*>(slots + NP * SLOT);
     uint64_t* full = bars;                 // [NP] plane staged (BR_PROD*32 arrivals)
     uint64_t* empty = bars + BR_MAXNP;     // [NP] plane no longer read (MMA commit)
-    uint64_t* tfull = bars + 2 * BR_MAXNP; // [2] accumulator ready (MMA commit)
-    uint64_t* tempty = tfull + 2;          // [2] accumulator drained (BR_EPI*32 arrivals)
-    uint64_t* drain = tempty + 2;          // [1] every MMA of the CTA done (teardown)
+    uint64_t* tfull = bars + 2 * BR_MAXNP; // [BR_OUT] output plane complete (MMA commit)
+    uint64_t* tempty = tfull + BR_OUT;     // [BR_OUT] output plane drained and cleared (BR_EPI*32 arrivals)
+    uint64_t* drain = tempty + BR_OUT;     // [1] every MMA of the CTA done (teardown)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
     int* s_fail = reinterpret_cast<int*>(tmem_slot + 1);
     const uint32_t ncols = brick_tmem_cols(A, coutp);
     const int mma_warp = BR_PROD;
 
-    // weights of every tap (output channels co0..) in the canonical B layout: rows co at
-    // 16 B, 8-row groups 128 B apart, one region of coutp rows per 8 input channels
+    // weights of every tap (output channels co0..) in the canonical B layout: rows at 16 B, 8-row groups
+    // 128 B apart; per (dy, dx) and 8 input channels a region of 3 coutp rows, dz = +1, 0, -1
     for (int q = tid; q < 27 * coutp * nhg; q += BR_NT) {
         const int t = q / (coutp * nhg), r = q % (coutp * nhg), n = r / nhg, hg = r % nhg;
-        cp_async16(sm_u32(wsm) + (uint32_t)(((t * nhg + hg) * coutp + n) * 16),
+        cp_async16(sm_u32(wsm) + (uint32_t)(((((t % 9) * nhg + hg) * 3 + 2 - t / 9) * coutp + n) * 16),
                    a.w + ((size_t)(co0 + n) * 27 + t) * cin + hg * 8, true);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -392,7 +216,7 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
             nn_mbar_init(&full[i], BR_PROD * 32);
             nn_mbar_init(&empty[i], 1);
         }
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < BR_OUT; ++i) {
             nn_mbar_init(&tfull[i], 1);
             nn_mbar_init(&tempty[i], BR_EPI * 32);
         }
@@ -405,6 +229,14 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (warp > mma_warp) { // every output plane starts at zero
+        for (int c0 = 0; c0 < BR_OUT * A * coutp; c0 += 16)
+            tmem_zero16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0);
+        tmem_wait_st();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
 
     const int bw = 8 * A;
     const int bx = (nx + bw - 1) / bw, by = (ny + 15) / 16, nzc = (nz + zchunk - 1) / zchunk;
@@ -417,7 +249,7 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
         // waited for, fenced towards the tensor core's proxy and announced, so that one plane's
         // copies are always in flight while the previous one is published.
         unsigned pc = 0;          // planes staged so far (ring position)
-        const int K = NP - 3;     // planes whose copies stay in flight (3 slots are being read)
+        const int K = min(NP - 1, 5); // planes whose copies stay in flight (one slot is being read)
         int pend[BR_MAXNP] = {}, np_ = 0, ph = 0; // committed, not yet announced slots (oldest at ph)
         const uint32_t inv_h = (65536u + nhg - 1) / nhg; // q / nhg by a multiply, exact for q < 4096
         // wait until at most n copy groups of this thread are pending
@@ -479,64 +311,53 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
     } else if (warp == mma_warp) {
         // ---------------- MMA issuer (one warp, its elected lane issues) ----------------
         const uint32_t leader = elect_one();
-        const uint32_t idesc = idesc_bf16(CONV_TM, coutp);
-        const uint64_t bbase = kdesc(sm_u32(wsm), (uint32_t)(coutp * 16), 128u);
+        const uint64_t bbase = kdesc(sm_u32(wsm), (uint32_t)(3 * coutp * 16), 128u);
         const uint32_t bhi = (uint32_t)(bbase >> 32), tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
-        unsigned pc = 0, pw = 0; // planes waited for, output planes done
+        unsigned pc = 0, on = 0; // planes waited for, output planes of the bricks before this one
         for (int br = blockIdx.x; br < nbricks && !fail; br += gridDim.x) {
             const int zc = br / (bx * by);
             const int z0 = zc * zchunk, z1 = min(nz, z0 + zchunk);
-            const unsigned pfirst = pc; // ring position of plane z0 - 1
-            auto wait_full = [&](unsigned p) {
-                return __all_sync(0xffffffffu, nn_mbar_wait(&full[p % NP], (p / NP) & 1u)) != 0;
-            };
-            for (int k = 0; k < 2 && !fail; ++k, ++pc)
-                if (!wait_full(pc)) fail = true;
-            for (int z = z0; z < z1 && !fail; ++z, ++pw) {
-                if (!wait_full(pc)) { // plane z + 1
+            for (int p = z0 - 1; p <= z1 && !fail; ++p, ++pc) {
+                if (!__all_sync(0xffffffffu, nn_mbar_wait(&full[pc % NP], (pc / NP) & 1u))) {
                     fail = true;
                     break;
                 }
-                ++pc;
-                const int tb = (int)(pw & 1u);
-                if (pw >= 2 && !__all_sync(0xffffffffu, nn_mbar_wait(&tempty[tb], ((pw / 2) - 1) & 1u))) {
+                // the output planes that p contributes to; p + 1 is new: its place must be cleared
+                const int zlo = max(z0, p - 1), zhi = min(z1 - 1, p + 1);
+                const unsigned olo = on + (unsigned)(zlo - z0), ohi = on + (unsigned)(zhi - z0);
+                if (zhi == p + 1 && ohi >= (unsigned)BR_OUT &&
+                    !__all_sync(0xffffffffu, nn_mbar_wait(&tempty[ohi % BR_OUT], (ohi / BR_OUT - 1) & 1u))) {
                     fail = true;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t dacc = tmem_u + (uint32_t)(tb * A * coutp);
-                // descriptors differ only in their start address (bits 0-13, in 16-byte
-                // units): one base per operand, offsets added
-                for (int dz = -1; dz <= 1; ++dz) {
-                    const unsigned pr = pfirst + (unsigned)(z - z0 + 1 + dz); // ring position of plane z + dz
-                    const uint64_t abase = kdesc(sm_u32(slots + (size_t)(pr % NP) * SLOT), (uint32_t)REG,
-                                                 (uint32_t)(W * 16));
-                    const uint32_t ahi = (uint32_t)(abase >> 32);
-                    const int tz = (dz + 1) * 9;
+                const uint64_t abase = kdesc(sm_u32(slots + (size_t)(pc % NP) * SLOT), (uint32_t)REG, (uint32_t)(W * 16));
+                const uint32_t ahi = (uint32_t)(abase >> 32);
+                // runs of output planes at consecutive places of the ring
+                for (unsigned o = olo; o <= ohi;) {
+                    const unsigned cnt = min(ohi - o + 1, (unsigned)BR_OUT - o % BR_OUT);
+                    const int blk = (int)(o - olo) + zlo - (p - 1); // first weight block (dz = +1, 0, -1)
+                    const uint32_t idesc = idesc_bf16(CONV_TM, (int)cnt * coutp);
+                    const uint32_t dacc = tmem_u + (o % BR_OUT) * (uint32_t)coutp;
                     for (int s2 = 0; s2 < cin / 16; ++s2) {
                         const uint32_t a_s = (uint32_t)abase + (uint32_t)(2 * s2 * (REG >> 4));
-                        const uint32_t b_s = (uint32_t)bbase + (uint32_t)(2 * s2 * coutp + tz * nhg * coutp);
+                        const uint32_t b_s = (uint32_t)bbase + (uint32_t)((2 * s2 * 3 + blk) * coutp);
 #pragma unroll
                         for (int tyx = 0; tyx < 9; ++tyx) {
                             const int dy = tyx / 3, dx = tyx % 3; // 0..2: offsets + 1
-                            const uint32_t bd = b_s + (uint32_t)(tyx * nhg * coutp);
-                            // every tile's first product of the plane overwrites its accumulator
-                            const uint32_t acc = (dz > -1 || s2 > 0 || tyx > 0) ? 1u : 0u;
+                            const uint32_t bd = b_s + (uint32_t)(tyx * nhg * 3 * coutp);
 #pragma unroll
                             for (int j = 0; j < A; ++j)
-                                umma_bf16_warp(dacc + (uint32_t)(j * coutp), a_s + (uint32_t)(dy * W + dx + 8 * j), ahi,
-                                               bd, bhi, idesc, acc, leader);
+                                umma_bf16_warp(dacc + (uint32_t)(j * BR_OUT * coutp), a_s + (uint32_t)(dy * W + dx + 8 * j),
+                                               ahi, bd, bhi, idesc, 1u, leader);
                         }
                     }
+                    o += cnt;
                 }
-                umma_commit_warp(&tfull[tb], leader);
-                // plane z - 1 is read by no later output plane of this brick
-                umma_commit_warp(&empty[(pfirst + (unsigned)(z - z0)) % NP], leader);
+                umma_commit_warp(&empty[pc % NP], leader);
+                if (p > z0) umma_commit_warp(&tfull[(on + (unsigned)(p - 1 - z0)) % BR_OUT], leader); // plane p - 1
             }
-            if (!fail) { // the brick's last two planes (z1 - 1, z1) are released too
-                umma_commit_warp(&empty[(pfirst + (unsigned)(z1 - z0)) % NP], leader);
-                umma_commit_warp(&empty[(pfirst + (unsigned)(z1 - z0 + 1)) % NP], leader);
-            }
+            on += (unsigned)(z1 - z0);
         }
         if (fail && lane == 0) atomicExch(s_fail, 1);
     } else {
@@ -549,9 +370,9 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
             const int x0 = (col % bx) * bw, y0 = (col / bx) * 16;
             const int z0 = zc * zchunk, z1 = min(nz, z0 + zchunk);
             for (int z = z0; z < z1 && !fail; ++z, ++pw) {
-                const int tb = (int)(pw & 1u);
+                const int tb = (int)(pw % BR_OUT);
                 // one lane waits, the warp follows (the TMEM loads below are warp-collective)
-                bool ok = lane == 0 ? nn_mbar_wait(&tfull[tb], (pw / 2) & 1u) : true;
+                bool ok = lane == 0 ? nn_mbar_wait(&tfull[tb], (pw / BR_OUT) & 1u) : true;
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                 if (!ok) {
                     fail = true;
@@ -564,7 +385,10 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
                     const size_t v = ((size_t)z * ny + gy) * nx + gx;
                     for (int c0 = 0; c0 < coutp; c0 += 16) {
                         float acc[16];
-                        tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(tb * A * coutp + j * coutp + c0), acc);
+                        const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((j * BR_OUT + tb) * coutp + c0);
+                        __syncwarp(); // (the loads are warp-collective)
+                        tmem_ld16(at, acc);
+                        tmem_zero16(at);
                         if (!vin) continue;
                         const int cg = co0 + c0; // channel in the full output
                         if (a.bias)
@@ -599,6 +423,8 @@ __global__ void __launch_bounds__(BR_NT, 1) conv3d_brick_kernel(const ConvArgs a
                         }
                     }
                 }
+                __syncwarp();
+                tmem_wait_st();
                 tc_fence_before();
                 nn_mbar_arrive(&tempty[tb]);
             }

@@ -203,20 +203,17 @@ class WarmStartNet {
         a.relu = relu;
         a.y_f32 = y_f32;
         a.err = err;
-        // brick kernel (halo staged once per plane) when a geometry fits: the output channels
-        // in as few launches as possible (1, 2 or 4), then two or one M-tiles per brick, then
-        // four or three plane slots
-        // More M-tiles per brick (A) give the tensor core more independent accumulators to
-        // interleave; no wider than the grid.
+        // The output channels in as few launches as possible, then the most M-tiles per brick (independent
+        // accumulators for the tensor core to interleave; no wider than the grid, TMEM allowing), then the most
+        // plane slots; two slots (one read, one loading) only where half the tiles do not have three.
         int amax = 1;
         while (amax < 8 && 8 * amax * 2 <= std::max(8, d.nx)) amax *= 2;
-        for (int split = 1; split <= 4; split *= 2)
+        for (int coutp = cout; coutp >= 16; coutp -= 16)
             for (int A = amax; A >= 1; A /= 2)
-                for (int NP = 8; NP >= 3; --NP) { // 3 slots read, NP - 3 loading ahead
-                    const int coutp = cout / split;
-                    if (cout % split || coutp % 16 || cin > 128) continue;
-                    if (brick_smem(A, NP, cin, coutp) > kBrickSmemMax || 2 * A * coutp > 512) continue;
-                    if (A > 1 && NP < 5 && brick_smem(A / 2, 5, cin, coutp) <= kBrickSmemMax) continue; // keep lookahead
+                for (int NP = BR_MAXNP; NP >= 2; --NP) {
+                    if (cout % coutp || 3 * coutp > 256 || BR_OUT * A * coutp > 512) continue;
+                    if (brick_smem(A, NP, cin, coutp) > kBrickSmemMax) continue;
+                    if (A > 1 && NP < 3 && brick_smem(A / 2, 3, cin, coutp) <= kBrickSmemMax) continue; // keep lookahead
                     auto kern = A == 8 ? conv3d_brick_kernel<8>
                               : A == 4 ? conv3d_brick_kernel<4>
                               : A == 2 ? conv3d_brick_kernel<2> : conv3d_brick_kernel<1>;
@@ -229,28 +226,13 @@ class WarmStartNet {
                     g.zchunk = brick_zchunk(cols, d.nz, num_sms());
                     const long long bricks = (long long)cols * ((d.nz + g.zchunk - 1) / g.zchunk);
                     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(bricks, num_sms()));
-                    for (int c = 0; c < split; ++c) {
-                        g.co0 = c * coutp;
+                    for (g.co0 = 0; g.co0 < cout; g.co0 += coutp) {
                         kern<<<grid, BR_NT, brick_smem(A, NP, cin, coutp), s>>>(a, g);
                         MF3D_LAUNCH_CK();
                     }
                     return;
                 }
-        const size_t smem = conv_smem(cin, cout);
-        MF3D_CK(cudaFuncSetAttribute(conv3d_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)conv_smem(CONV_MAXC, CONV_MAXC)));
-        // all of the unified L1 as shared memory: without it the driver sizes the carveout for
-        // the largest allowed allocation and keeps one CTA per SM
-        MF3D_CK(cudaFuncSetAttribute(conv3d_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared));
-        int occ = 0;
-        MF3D_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, conv3d_tc_kernel, CONV_NT, smem));
-        // no more CTAs per SM than their TMEM accumulators fit in (512 columns)
-        occ = std::max(1, std::min<int>(occ, (int)(512 / tmem_cols(cout))));
-        const long long tiles = ((long long)d.v() + CONV_TM - 1) / CONV_TM;
-        const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(tiles, (long long)occ * num_sms()));
-        conv3d_tc_kernel<<<grid, CONV_NT, smem, s>>>(a);
-        MF3D_LAUNCH_CK();
+        throw Error(MF3D_E_INVALID, "convolution does not fit in shared memory");
     }
 
     // Launch shape of the weight gradient of one layer.

@@ -231,3 +231,19 @@ def test_shipped_weights_beat_the_linear_guess(mf3d):
     assert float((hw.reshape(-1) - h).abs().max()) < 1e-4  # the same head (h is stored in FP32)
     s.close()
     ws.close()
+
+
+# one shape per way the output planes meet the ring of four in TMEM (bricks of 2, 3, 4, 5 and many planes, one
+# brick and several), ragged tiles in x and y, and channel counts that need one, two and more launches
+@pytest.mark.parametrize("shape", [(2, 16, 8), (3, 17, 9), (4, 5, 64), (5, 33, 70), (37, 16, 24), (1, 1, 1)])
+@pytest.mark.parametrize("cin,cout", [(16, 16), (48, 16), (32, 32), (64, 64), (128, 64), (128, 128), (112, 48)])
+def test_conv3d_ring_and_channel_splits_vs_oracle(mf3d, shape, cin, cout):
+    """Products of BF16 values accumulated in FP32 over 27 cin terms: 2e-5 of the largest output, as above."""
+    M = mf3d
+    r = np.random.default_rng(cin * 31 + cout + sum(shape))
+    nz, ny, nx = shape
+    x = _bf(r.normal(size=(nz * ny * nx, cin)))
+    w = _bf(r.normal(size=(cout, 27, cin)) / np.sqrt(27 * cin))
+    y = M.nn_conv3d(M.Grid3D(nx, ny, nz, 1.0), x, w, None, out_f32=True)
+    ref = N.conv3d(_np(x).reshape(nz, ny, nx, cin), _np(w)).reshape(-1, cout)
+    assert _rel(_np(y), ref) < 2e-5
