@@ -312,8 +312,9 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
         const long long l0 = g_launches;
         for (int r = 0; r < R; ++r) {
             HeadSolver& H = *hs_[r];
-            copy_h_[r] = CopyItem{(x0 && x0[r]) ? x0[r] : H.x0_.as<double>(), H.x_.as<double>(), H.G_[0].n};
-            copy_h_[R + r] = CopyItem{H.x_.as<double>(), h[r], H.G_[0].n};
+            const Guess g = make_guess(to_dev(H.bc_));
+            copy_h_[r] = CopyItem{x0 ? x0[r] : nullptr, H.x_.as<double>(), H.G_[0].n, H.G_[0].nx, g};
+            copy_h_[R + r] = CopyItem{H.x_.as<double>(), h[r], H.G_[0].n, H.G_[0].nx, g};
         }
         MF3D_CK(cudaEventRecord(ev0_, s_));
         MF3D_CK(cudaMemcpyAsync(copy_d_, copy_h_, 2 * R * sizeof(CopyItem), cudaMemcpyHostToDevice, s_));
@@ -697,7 +698,7 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
                                             flexible_ ? 1 : 0, cfg_.cg_rtol, kSolveBudgetNs, SOLVE_PCG_MG,
                                             cfg_.cg_max_iter + 1);
         MF3D_LAUNCH_CK();
-        batch_residual_kernel<<<pgrid(tot3_), dim3(32, 8), 0, s>>>(items_d_, off3_d_, R, tot3_, 0,
+        batch_residual_kernel<<<pgrid(tot3_), dim3(32, 8), 0, s>>>(items_d_, copy_d_ + R, off3_d_, R, tot3_, 0,
                                                                    cfg_.conv_norm == MF3D_CONV_B ? 1 : 0);
         MF3D_LAUNCH_CK();
         batch_gate_kernel<<<1, 256, 0, s>>>(items_d_, R, ctl_d_, cond_, with_cond ? 1 : 0, 0, any_d_);
@@ -720,12 +721,10 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
 
     void record_post(cudaStream_t s) {
         const int R = (int)hs_.size();
-        batch_xfinish_kernel<<<pgrid(tot1_), PK_NT, 0, s>>>(items_d_, off1_d_, R, tot1_);
+        batch_xfinish_kernel<<<pgrid(tot1_), PK_NT, 0, s>>>(items_d_, copy_d_ + R, off1_d_, R, tot1_);
         MF3D_LAUNCH_CK();
-        batch_residual_kernel<<<pgrid(tot3_), dim3(32, 8), 0, s>>>(items_d_, off3_d_, R, tot3_, 1,
+        batch_residual_kernel<<<pgrid(tot3_), dim3(32, 8), 0, s>>>(items_d_, copy_d_ + R, off3_d_, R, tot3_, 1,
                                                                    cfg_.conv_norm == MF3D_CONV_B ? 1 : 0);
-        MF3D_LAUNCH_CK();
-        batch_copy_kernel<<<pgrid(tot1_), PK_NT, 0, s>>>(copy_d_ + R, off1_d_, R, tot1_);
         MF3D_LAUNCH_CK();
         batch_states_kernel<<<1, 256, 0, s>>>(items_d_, R, states_d_, errs_d_);
         MF3D_LAUNCH_CK();

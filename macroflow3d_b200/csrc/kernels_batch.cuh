@@ -9,6 +9,7 @@
 // a grid of a few CTAs per SM walks the virtual blocks.
 #pragma once
 #include "kernels_pcg.cuh"
+#include "kernels_setup.cuh"
 
 namespace mf3d {
 
@@ -40,9 +41,11 @@ struct BatchCtl {
 };
 
 struct CopyItem {
-    const double* src;
+    const double* src; // null: the initial guess g on rows of nx cells
     double* dst;
     size_t n;
+    int nx;
+    Guess g;
 };
 
 // PCG state initialisation of every realisation (one thread each); tickets cleared.
@@ -101,26 +104,27 @@ __global__ void batch_gate_kernel(const PcgItem* __restrict__ items, int R, Batc
     }
 }
 
-// dst = src for every item (one segment per realisation)
+// dst = src (or the initial guess) for every item (one segment per realisation)
 __global__ void __launch_bounds__(PK_NT) batch_copy_kernel(const CopyItem* __restrict__ items,
                                                            const int* __restrict__ off, int nseg, int total) {
     for (int b = blockIdx.x; b < total; b += gridDim.x) {
         const int s = find_seg(off, nseg, b);
         const CopyItem it = items[s];
         const int o = __ldg(off + s), cnt = __ldg(off + s + 1) - o;
-        for (size_t c = (size_t)(b - o) * PK_NT + threadIdx.x; c < it.n; c += (size_t)cnt * PK_NT) it.dst[c] = it.src[c];
+        for (size_t c = (size_t)(b - o) * PK_NT + threadIdx.x; c < it.n; c += (size_t)cnt * PK_NT) it.dst[c] = it.src ? it.src[c] : guess_at(it.g, (int)(c % it.nx), it.nx);
     }
 }
 
-// r = b - A x with norms: mode 0 at the start of the solves, 1 (true residual) at the end.
+// r = b - A x with norms: mode 0 at the start of the solves, 1 (true residual of the finished head) at the end.
 __global__ void __launch_bounds__(PK_NT) batch_residual_kernel(const PcgItem* __restrict__ items,
+                                                               const CopyItem* __restrict__ heads,
                                                                const int* __restrict__ off, int nseg, int total,
                                                                int mode, int ref_is_b) {
     for (int b = blockIdx.x; b < total; b += gridDim.x) {
         const int s = find_seg(off, nseg, b);
         const PcgItem& it = items[s];
         const VBlk vb = make_vblk(b - __ldg(off + s), it.cgx, it.cgy, it.cgz);
-        residual_body<double>(it.L, it.x, it.b, mode == 0 ? it.r : it.Ap, it.st, it.partials, it.tickets + 2, mode,
+        residual_body<double>(it.L, mode == 0 ? it.x : heads[s].dst, it.b, mode == 0 ? it.r : it.Ap, it.st, it.partials, it.tickets + 2, mode,
                               ref_is_b, mode == 0 ? it.r32 : nullptr, 0, 0, it.zchunk, vb);
     }
 }
@@ -153,13 +157,14 @@ __global__ void __launch_bounds__(PK_NT) batch_xr_update_kernel(const PcgItem* _
     }
 }
 
-// the steps that the heads do not hold yet, after the loop
+// the heads with the steps that x does not hold yet, into the copies' destinations, after the loop
 __global__ void __launch_bounds__(PK_NT) batch_xfinish_kernel(const PcgItem* __restrict__ items,
+                                                              const CopyItem* __restrict__ to,
                                                               const int* __restrict__ off, int nseg, int total) {
     for (int b = blockIdx.x; b < total; b += gridDim.x) {
         const int s = find_seg(off, nseg, b), o = __ldg(off + s);
         const PcgItem& it = items[s];
-        xfinish_body(it.n, it.x, it.p, it.p2, it.st, b - o, __ldg(off + s + 1) - o);
+        xfinish_body(it.n, it.x, it.p, it.p2, it.st, to[s].dst, b - o, __ldg(off + s + 1) - o);
     }
 }
 

@@ -406,23 +406,25 @@ __global__ void __launch_bounds__(PMV_TX * PMV_TY, MF3D_PMATVEC_MINB)
     pmatvec_body<TZ>(L, z, p0, p1, Ap, x, st, partials, ticket, zchunk, hw_vblk(), pmv_sm);
 }
 
-// The steps that x does not hold yet (at most two, see pmatvec_body), after the loop.
-__device__ __forceinline__ void xfinish_body(size_t n, double* __restrict__ x, const double* __restrict__ p0,
-                                             const double* __restrict__ p1, const PcgState* st, int blk, int nblk) {
-    const int it = st->iter, left = it - st->x_done;
-    if (st->solver == SOLVE_MG || left < 1 || left > 2) return;
+// out = x with the steps that it does not hold yet (at most two, see pmatvec_body), after the loop.
+__device__ __forceinline__ void xfinish_body(size_t n, const double* __restrict__ x, const double* __restrict__ p0,
+                                             const double* __restrict__ p1, const PcgState* st,
+                                             double* __restrict__ out, int blk, int nblk) {
+    const int it = st->iter, left = st->solver == SOLVE_MG ? 0 : it - st->x_done;
     const double a1 = st->alpha, a0 = st->alpha_prev;
     const double* pa = ((it - 1) & 1) ? p0 : p1; // p_{it-1}: pcg_pbuf_out(it - 1)
     const double* pb = ((it - 1) & 1) ? p1 : p0; // p_{it-2}
     for (size_t c = blk * (size_t)PK_NT + threadIdx.x; c < n; c += (size_t)nblk * PK_NT) {
         double v = x[c];
         if (left == 2) v = v + a0 * pb[c];
-        x[c] = v + a1 * pa[c];
+        if (left >= 1) v = v + a1 * pa[c];
+        out[c] = v;
     }
 }
-__global__ void __launch_bounds__(PK_NT) xfinish_kernel(size_t n, double* __restrict__ x, const double* __restrict__ p0,
-                                                        const double* __restrict__ p1, const PcgState* st) {
-    xfinish_body(n, x, p0, p1, st, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(PK_NT) xfinish_kernel(size_t n, const double* __restrict__ x,
+                                                        const double* __restrict__ p0, const double* __restrict__ p1,
+                                                        const PcgState* st, double* __restrict__ out) {
+    xfinish_body(n, x, p0, p1, st, out, blockIdx.x, gridDim.x);
 }
 
 // r -= alpha Ap (alpha = rho_new / pAp); ||r||^2 and, for the flexible form,

@@ -101,21 +101,6 @@ __device__ __forceinline__ void cell_coefs(const LevelOp<TC>& L, int i, int j, i
 // Deterministic grid-wide sum: every block writes its partial, the last block to arrive
 // adds the partials in index order.  `ticket` must start at 0; it is reset by the last block.
 // ---------------------------------------------------------------------------------------
-template <int NT>
-__device__ __forceinline__ double block_sum(double v, double* red /* NT/32 doubles */) {
-    const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int w = tid >> 5, l = tid & 31;
-    if (l == 0) red[w] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (tid == 0) {
-        for (int i = 0; i < NT / 32; ++i) s += red[i];
-    }
-    __syncthreads();
-    return s; // valid on thread 0
-}
-
 // Returns true on thread 0 of the last block to finish; `out` then holds the grid sums.
 // Blocks may be 1-, 2- or 3-D; NT is the number of threads per block.  `bid` is the block's
 // index among the `nblocks` that share the partials (the hardware block index by default; a

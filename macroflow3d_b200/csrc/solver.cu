@@ -328,12 +328,22 @@ struct CoefStore {
     }
 };
 
+template <class TC> static FacePtrs<TC> face_ptrs(const LevelOp<TC>& L) {
+    return {(TC*)L.cx, (TC*)L.cy, (TC*)L.cz, (TC*)L.bxm, (TC*)L.bym, (TC*)L.bzm};
+}
+// the FP64 set (null: none) and a second one (null: none) of a level
 template <class TC>
-static void launch_faces(cudaStream_t s, const Geom& G, const double* K, const mf3d_bc& bc, double scale,
-                         const LevelOp<TC>& L) {
+static void launch_faces(cudaStream_t s, const Geom& G, const double* K, const mf3d_bc& bc,
+                         const LevelOp<double>* A, double scale, const LevelOp<TC>* B) {
     const ColLaunch cl = col_launch(G.nx, G.ny, G.nz);
-    faces_kernel<TC><<<cl.grid, cl.block, 0, s>>>(G.nx, G.ny, G.nz, K, to_dev(bc), scale, (TC*)L.cx, (TC*)L.cy,
-                                                  (TC*)L.cz, (TC*)L.bxm, (TC*)L.bym, (TC*)L.bzm, cl.zchunk);
+    faces_kernel<double, TC><<<cl.grid, cl.block, 0, s>>>(G.nx, G.ny, G.nz, K, to_dev(bc), scale,
+                                                          A ? face_ptrs(*A) : FacePtrs<double>{},
+                                                          B ? face_ptrs(*B) : FacePtrs<TC>{}, cl.zchunk);
+    MF3D_LAUNCH_CK();
+}
+static void launch_guess(cudaStream_t s, const Geom& G, const mf3d_bc& bc, double* h) {
+    const size_t nrows = (size_t)G.ny * G.nz;
+    guess_kernel<<<grid1d(nrows * 32, 256), 256, 0, s>>>(G.nx, nrows, make_guess(to_dev(bc)), h);
     MF3D_LAUNCH_CK();
 }
 
@@ -374,7 +384,9 @@ static mf3d_kernel_timing timing(const char* name, float ms, double bytes, int p
 
 struct VCycleBase {
     virtual ~VCycleBase() {}
-    virtual void build_coefs(cudaStream_t s, const std::vector<const double*>& Klev) = 0;
+    // op64[l]: the FP64 coefficients of level l to build as well, or null
+    virtual void build_coefs(cudaStream_t s, const std::vector<const double*>& Klev,
+                             const std::vector<const LevelOp<double>*>& op64) = 0;
     // z (type T) = V-cycle of the level-0 right-hand side bound at construction; when
     // rho_out != null, <r64, z> is summed into *rho_out.
     virtual void run(cudaStream_t s, void* z, double* rho_out) = 0;
@@ -835,9 +847,13 @@ template <class T, class TC> class VCycle : public VCycleBase {
     int pre() const { return pre_; }
     int post() const { return post_; }
 
-    void build_coefs(cudaStream_t s, const std::vector<const double*>& Klev) override {
-        if (!std::is_same<TC, double>::value)
-            for (int l = 0; l < Lt_; ++l) launch_faces<TC>(s, G_[l], Klev[l], bc_, scale_[l], ops_[l]);
+    void build_coefs(cudaStream_t s, const std::vector<const double*>& Klev,
+                     const std::vector<const LevelOp<double>*>& op64) override {
+        for (int l = 0; l < (int)G_.size(); ++l) {
+            const bool own = l < Lt_ && !std::is_same<TC, double>::value;
+            if (op64[l] || own)
+                launch_faces<TC>(s, G_[l], Klev[l], bc_, op64[l], own ? scale_[l] : 1.0, own ? &ops_[l] : nullptr);
+        }
         size_t wo = 0;
         for (int l = Lw_; l < (int)G_.size(); ++l) {
             tail_weights_kernel<<<grid1d(G_[l].n, 256), 256, 0, s>>>(op64_[l], tail_w_->as<double>() + wo);
@@ -1596,7 +1612,6 @@ class HeadSolver {
         vec(p_);
         vec(p2_);
         vec(Ap_);
-        vec(x0_);
         // reduction scratch sized for the largest grid any reduction uses
         size_t cap = std::max<size_t>((size_t)grid1d(n, PK_NT) * 2, col_launch(G_[0].nx, G_[0].ny, G_[0].nz).nblocks) + 1024;
         {
@@ -1666,23 +1681,24 @@ class HeadSolver {
         if (!K) throw Error(MF3D_E_INVALID, "K is null");
         const long long l0 = g_launches;
         const int nl = (int)G_.size();
+        // (a copy first: the caller may free or reuse K on another stream once this returns)
         MF3D_CK(cudaMemcpyAsync(Klev_[0]->p, K, G_[0].n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        std::vector<const double*> Kp(nl, Klev_[0]->as<double>());
         for (int l = 0; l + 1 < nl; ++l) {
             const Geom& c = G_[l + 1];
             const ColLaunch cl = col_launch(c.nx, c.ny, c.nz);
-            coarsen_kernel<<<cl.grid, cl.block, 0, s>>>(c.nx, c.ny, c.nz, Klev_[l]->as<double>(),
-                                                        Klev_[l + 1]->as<double>(), cl.zchunk);
+            coarsen_kernel<<<cl.grid, cl.block, 0, s>>>(c.nx, c.ny, c.nz, Kp[l], Klev_[l + 1]->as<double>(), cl.zchunk);
             MF3D_LAUNCH_CK();
+            Kp[l + 1] = Klev_[l + 1]->as<double>();
         }
-        std::vector<const double*> Kp(nl);
-        for (int l = 0; l < nl; ++l) Kp[l] = Klev_[l]->as<double>();
+        std::vector<const LevelOp<double>*> o64(nl, nullptr);
         for (int l = 0; l < nl; ++l)
-            if (coef64_[l]) launch_faces<double>(s, G_[l], Kp[l], bc_, 1.0, op64_[l]);
-        vc_->build_coefs(s, Kp);
+            if (coef64_[l]) o64[l] = &op64_[l];
+        vc_->build_coefs(s, Kp, o64);
         {
             const ColLaunch cl = col_launch(G_[0].nx, G_[0].ny, G_[0].nz);
-            rhs_guess_kernel<<<cl.grid, cl.block, 0, s>>>(G_[0].nx, G_[0].ny, G_[0].nz, G_[0].dx, Kp[0], to_dev(bc_),
-                                                          b_.as<double>(), x0_.as<double>(), cl.zchunk);
+            rhs_kernel<<<cl.grid, cl.block, 0, s>>>(G_[0].nx, G_[0].ny, G_[0].nz, G_[0].dx, Kp[0], to_dev(bc_),
+                                                    b_.as<double>(), cl.zchunk);
         }
         MF3D_LAUNCH_CK();
         setup_launches_ = (int)(g_launches - l0);
@@ -1735,7 +1751,8 @@ class HeadSolver {
         const long long l0 = g_launches;
         body_runs_ = 0;
         MF3D_CK(cudaEventRecord(ev0_, s));
-        MF3D_CK(cudaMemcpyAsync(x_.p, x0 ? x0 : x0_.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        if (x0) MF3D_CK(cudaMemcpyAsync(x_.p, x0, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        else launch_guess(s, G_[0], bc_, x_.as<double>());
         MF3D_CK(cudaMemsetAsync(tickets_.p, 0, tickets_.bytes, s));
         const bool mg = cfg_.solver == MF3D_SOLVER_MG, cg = cfg_.solver == MF3D_SOLVER_CG;
         pcg_init_kernel<<<1, 1, 0, s>>>(state_.as<PcgState>(), mg ? cfg_.mg_max_cycles : cfg_.cg_max_iter,
@@ -1758,13 +1775,10 @@ class HeadSolver {
                 if (host_state_->stop) break;
             }
         }
-        if (!mg) {
-            xfinish_kernel<<<grid1d(n, PK_NT), PK_NT, 0, s>>>(n, x_.as<double>(), p_.as<double>(), p2_.as<double>(),
-                                                              state_.as<PcgState>());
-            MF3D_LAUNCH_CK();
-        }
-        launch_residual(s, 1);
-        MF3D_CK(cudaMemcpyAsync(h, x_.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        xfinish_kernel<<<grid1d(n, PK_NT), PK_NT, 0, s>>>(n, x_.as<double>(), p_.as<double>(), p2_.as<double>(),
+                                                          state_.as<PcgState>(), h);
+        MF3D_LAUNCH_CK();
+        launch_residual(s, 1, h);
         MF3D_CK(cudaEventRecord(ev1_, s));
         MF3D_CK(cudaMemcpyAsync(host_state_, state_.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
         MF3D_CK(cudaMemcpyAsync(host_state_ + 1, err_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1852,13 +1866,14 @@ class HeadSolver {
         MF3D_LAUNCH_CK();
     }
 
-    void launch_residual(cudaStream_t s, int mode) {
+    // mode 0: of x_, into r_; 1: of the head `x`, the norm only (into scratch)
+    void launch_residual(cudaStream_t s, int mode, const double* x = nullptr) {
         const size_t n = G_[0].n;
         double* out = mode == 0 ? r_.as<double>() : Ap_.as<double>();
         (void)n;
         const ColLaunch cl = col_launch(G_[0].nx, G_[0].ny, G_[0].nz);
         residual_kernel<double><<<cl.grid, cl.block, 0, s>>>(
-            op64_[0], x_.as<double>(), b_.as<double>(), out, state_.as<PcgState>(), partials_.as<double>(),
+            op64_[0], x ? x : x_.as<double>(), b_.as<double>(), out, state_.as<PcgState>(), partials_.as<double>(),
             tickets_.as<unsigned>() + 2, mode, cfg_.conv_norm == MF3D_CONV_B ? 1 : 0,
             mode == 1 ? nullptr : r32_.as<float>(), cond_, 0, cl.zchunk);
         MF3D_LAUNCH_CK();
@@ -1945,7 +1960,7 @@ class HeadSolver {
     std::vector<LevelOp<double>> op64_;
     std::vector<std::unique_ptr<CoefStore>> coef64_;
     std::vector<std::unique_ptr<DevMem>> Klev_;
-    DevMem x_, b_, r_, p_, p2_, Ap_, x0_, z_; // p_, p2_: search directions, alternating by iteration
+    DevMem x_, b_, r_, p_, p2_, Ap_, z_; // p_, p2_: search directions, alternating by iteration
     DevMem partials_, tickets_, state_, mb_, err_, r32_;
     std::unique_ptr<VCycleBase> vc_;
     PcgState* host_state_ = nullptr; // pinned: the state, then the pipelines' error flag
@@ -2340,7 +2355,7 @@ struct OneLevel {
         G = Geom{g->nx, g->ny, g->nz, (size_t)g->nx * g->ny * g->nz, g->dx};
         op = make_op<double>(G, *bc, pin != 0, 1.0);
         cs.build<double>(G, sizeof(double), op);
-        launch_faces<double>(s, G, K, *bc, 1.0, op);
+        launch_faces<double>(s, G, K, *bc, &op, 1.0, nullptr);
     }
 };
 
@@ -2516,19 +2531,10 @@ int mf3d_build_rhs(const mf3d_grid* g, const mf3d_bc* bc, const double* K, doubl
         const size_t n = (size_t)g->nx * g->ny * g->nz;
         (void)n;
         const ColLaunch cl = col_launch(g->nx, g->ny, g->nz);
-        rhs_guess_kernel<<<cl.grid, cl.block, 0, s>>>(g->nx, g->ny, g->nz, g->dx, K, to_dev(*bc), b, nullptr, cl.zchunk);
+        rhs_kernel<<<cl.grid, cl.block, 0, s>>>(g->nx, g->ny, g->nz, g->dx, K, to_dev(*bc), b, cl.zchunk);
         MF3D_LAUNCH_CK();
         MF3D_CK(cudaStreamSynchronize(s));
     });
-}
-
-__global__ void guess_kernel(int nx, int ny, int nz, BcDev bc, double* __restrict__ h) {
-    const size_t n = (size_t)nx * ny * nz;
-    const bool lin = bc.type[0] == BC_DIRICHLET && bc.type[1] == BC_DIRICHLET;
-    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(c % nx);
-        h[c] = lin ? bc.value[0] + (bc.value[1] - bc.value[0]) * (((double)i + 0.5) / (double)nx) : 0.0;
-    }
 }
 
 int mf3d_init_head_guess(const mf3d_grid* g, const mf3d_bc* bc, double* h, void* stream) {
@@ -2537,9 +2543,7 @@ int mf3d_init_head_guess(const mf3d_grid* g, const mf3d_bc* bc, double* h, void*
         need(bc, "bc");
         need(h, "h");
         cudaStream_t s = (cudaStream_t)stream;
-        const size_t n = (size_t)g->nx * g->ny * g->nz;
-        guess_kernel<<<grid1d(n, 256), 256, 0, s>>>(g->nx, g->ny, g->nz, to_dev(*bc), h);
-        MF3D_LAUNCH_CK();
+        launch_guess(s, Geom{g->nx, g->ny, g->nz, (size_t)g->nx * g->ny * g->nz, g->dx}, *bc, h);
         MF3D_CK(cudaStreamSynchronize(s));
     });
 }
