@@ -738,34 +738,63 @@ __global__ void flip_weights_kernel(const __nv_bfloat16* __restrict__ w, __nv_bf
 }
 
 // ---- pooling, upsampling with concatenation, and their gradients (C channels) ----
+// (8 channels per thread in all of them: 16-byte accesses)
+struct Bf8 {
+    float f[8];
+};
+__device__ __forceinline__ Bf8 bf8_load(const __nv_bfloat16* p) {
+    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
+    const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&raw);
+    Bf8 v;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v.f[i] = __bfloat162float(e[i]);
+    return v;
+}
+__device__ __forceinline__ void bf8_store(__nv_bfloat16* p, const Bf8& v) {
+    __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] = __float2bfloat16(v.f[i]);
+    *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(o);
+}
 // average of the 8 children; fine grid (nx, ny, nz) even
 __global__ void pool_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int nx, int ny,
                             int nz, int C) {
-    const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
-    const size_t n = (size_t)cx * cy * cz * C;
+    const int cx = nx / 2, cy = ny / 2, cz = nz / 2, Q = C / 8;
+    const size_t n = (size_t)cx * cy * cz * Q;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const int c = (int)(e % C);
-        const size_t P = e / C;
+        const int q = (int)(e % Q);
+        const size_t P = e / Q;
         const int I = (int)(P % cx), J = (int)((P / cx) % cy), K = (int)(P / ((size_t)cx * cy));
-        float s = 0.f;
+        Bf8 s{};
+#pragma unroll
         for (int d = 0; d < 8; ++d) {
             const int i = 2 * I + (d & 1), j = 2 * J + ((d >> 1) & 1), k = 2 * K + (d >> 2);
-            s += __bfloat162float(x[((size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k)) * C + c]);
+            const Bf8 v = bf8_load(x + ((size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k)) * C + 8 * q);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s.f[u] += v.f[u];
         }
-        y[e] = __float2bfloat16(s * 0.125f);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s.f[u] *= 0.125f;
+        bf8_store(y + P * C + 8 * q, s);
     }
 }
-// dx_acc[child] += dy[parent] / 8
-__global__ void pool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ dx_acc, int nx, int ny,
-                                int nz, int C) {
-    const size_t n = (size_t)nx * ny * nz * C;
-    const int cx = nx / 2, cy = ny / 2;
+// Gradient of an encoder level's output from its two uses, times its ReLU derivative:
+// g[v] = (skip[v] + dy[parent] / 8) where act[v] > 0, summed in FP32
+__global__ void skip_pool_bwd_kernel(const __nv_bfloat16* __restrict__ skip, const __nv_bfloat16* __restrict__ dy,
+                                     const __nv_bfloat16* __restrict__ act, __nv_bfloat16* __restrict__ g, int nx,
+                                     int ny, int nz, int C) {
+    const int cx = nx / 2, cy = ny / 2, Q = C / 8;
+    const size_t n = (size_t)nx * ny * nz * Q;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const int c = (int)(e % C);
-        const size_t v = e / C;
+        const int q = (int)(e % Q);
+        const size_t v = e / Q;
         const int i = (int)(v % nx), j = (int)((v / nx) % ny), k = (int)(v / ((size_t)nx * ny));
         const size_t P = (size_t)(i >> 1) + (size_t)cx * ((size_t)(j >> 1) + (size_t)cy * (k >> 1));
-        dx_acc[e] += 0.125f * __bfloat162float(dy[P * C + c]);
+        const Bf8 s = bf8_load(skip + v * C + 8 * q), d = bf8_load(dy + P * C + 8 * q), a = bf8_load(act + v * C + 8 * q);
+        Bf8 o;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) o.f[u] = a.f[u] > 0.f ? s.f[u] + 0.125f * d.f[u] : 0.f;
+        bf8_store(g + v * C + 8 * q, o);
     }
 }
 // cat[v] = (coarse[parent(v)] (Ca channels), skip[v] (Cb channels)); fine grid (nx, ny, nz);
@@ -790,45 +819,43 @@ __global__ void upcat_kernel(const __nv_bfloat16* __restrict__ coarse, const __n
         reinterpret_cast<uint4*>(cat + v * (Ca + Cb))[q] = val;
     }
 }
-// gradient of upcat: dcoarse[P] = sum over the 8 children of dcat[child][0:Ca];
-// dskip_acc[v] += dcat[v][Ca:]
-__global__ void upcat_bwd_coarse_kernel(const __nv_bfloat16* __restrict__ dcat, float* __restrict__ dcoarse,
-                                        int nx, int ny, int nz, int Ca, int Cb) {
-    const int C = Ca + Cb, cx = nx / 2, cy = ny / 2, cz = nz / 2;
-    const size_t n = (size_t)cx * cy * cz * Ca;
+// Gradient of upcat: g[P] = (sum over the 8 children of dcat[child][0:Ca]) where act[P] > 0 (the ReLU derivative of
+// the coarse activation; FP32 sum), and skip[v] = dcat[v][Ca:], kept for the encoder.  One thread per coarse
+// cell and 8 channels of dcat: dcat is read once.
+__global__ void upcat_bwd_kernel(const __nv_bfloat16* __restrict__ dcat, const __nv_bfloat16* __restrict__ act,
+                                 __nv_bfloat16* __restrict__ g, __nv_bfloat16* __restrict__ skip, int nx, int ny,
+                                 int nz, int Ca, int Cb) {
+    const int C = Ca + Cb, cx = nx / 2, cy = ny / 2, cz = nz / 2, Q = C / 8, qa = Ca / 8;
+    const size_t n = (size_t)cx * cy * cz * Q;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const int c = (int)(e % Ca);
-        const size_t P = e / Ca;
+        const int q = (int)(e % Q);
+        const size_t P = e / Q;
         const int I = (int)(P % cx), J = (int)((P / cx) % cy), K = (int)(P / ((size_t)cx * cy));
-        float s = 0.f;
-        for (int d = 0; d < 8; ++d) {
+        auto child = [&](int d) {
             const int i = 2 * I + (d & 1), j = 2 * J + ((d >> 1) & 1), k = 2 * K + (d >> 2);
-            s += __bfloat162float(dcat[((size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k)) * C + c]);
+            return (size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k);
+        };
+        if (q < qa) {
+            Bf8 s{};
+#pragma unroll
+            for (int d = 0; d < 8; ++d) {
+                const Bf8 v = bf8_load(dcat + child(d) * C + 8 * q);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) s.f[u] += v.f[u];
+            }
+            const Bf8 a = bf8_load(act + P * Ca + 8 * q);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s.f[u] = a.f[u] > 0.f ? s.f[u] : 0.f;
+            bf8_store(g + P * Ca + 8 * q, s);
+        } else {
+#pragma unroll
+            for (int d = 0; d < 8; ++d) {
+                const size_t v = child(d);
+                *reinterpret_cast<uint4*>(skip + v * Cb + 8 * (q - qa)) = __ldg(reinterpret_cast<const uint4*>(dcat + v * C) + q);
+            }
         }
-        dcoarse[e] = s;
     }
 }
-__global__ void upcat_bwd_skip_kernel(const __nv_bfloat16* __restrict__ dcat, float* __restrict__ dskip_acc,
-                                      size_t V, int Ca, int Cb) {
-    const int C = Ca + Cb;
-    const size_t n = V * Cb;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const size_t v = e / Cb;
-        dskip_acc[e] += __bfloat162float(dcat[v * C + Ca + (e % Cb)]);
-    }
-}
-// g = bf16(acc * (act > 0)) (the ReLU derivative of a layer whose output gradient was summed
-// from two paths in FP32)
-__global__ void mask_to_bf16_kernel(const float* __restrict__ acc, const __nv_bfloat16* __restrict__ act,
-                                    __nv_bfloat16* __restrict__ g, size_t n) {
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
-        g[e] = __float2bfloat16(__bfloat162float(act[e]) > 0.f ? acc[e] : 0.f);
-}
-__global__ void bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ a, float* __restrict__ b, size_t n) {
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
-        b[e] = __bfloat162float(a[e]);
-}
-
 // ---- network input, output and loss ----
 // input channels: 0 lnK / 2, 1 the x-linear head guess - 1/2 (centred), 2..15 zero.
 // h_lin = h_w + (h_e - h_w) (i + 1/2) / nx (init_head_guess, solve_head.cu:56-73)

@@ -328,8 +328,7 @@ class WarmStartNet {
         float* lpart;
         // backward: gradient buffers (BF16 for the tensor-core operands, FP32 accumulators)
         __nv_bfloat16 *g0, *g1; // [V0 x 128] ping-pong gradient buffers, sized for the widest level use
-        float *acc0, *acc1, *acc2; // FP32 skip-gradient accumulators at L0 (16), L1 (32), L2 (64)
-        float* accc;               // FP32 coarse gradient of an upsampling (<= V1 x 64)
+        __nv_bfloat16 *sk0, *sk1, *sk2; // gradients of the skip connections at L0 (16), L1 (32), L2 (64)
         float* part;
         size_t part_floats;
     } bufs_;
@@ -374,10 +373,9 @@ class WarmStartNet {
         bufs_.lpart = f32(1024);
         bufs_.g0 = bf(V0 * 48);
         bufs_.g1 = bf(V0 * 48);
-        bufs_.acc0 = f32(V0 * 16);
-        bufs_.acc1 = f32(V1 * 32);
-        bufs_.acc2 = f32(V2 * 64);
-        bufs_.accc = f32(V1 * 64);
+        bufs_.sk0 = bf(V0 * 16);
+        bufs_.sk1 = bf(V1 * 32);
+        bufs_.sk2 = bf(V2 * 64);
         bufs_.part_floats = 0; // the largest layer's weight-gradient partials
         Dims dl[4] = {d, d.half(), d.half().half(), d.half().half().half()};
         for (const LayerSpec& L : kLayers)
@@ -401,15 +399,15 @@ class WarmStartNet {
         const Dims d1 = d0.half(), d2 = d1.half(), d3 = d2.half();
         layer(s, 0, d0, b.in, b.a0);
         layer(s, 1, d0, b.a0, b.e0);
-        pool_kernel<<<ew_grid(d1.v() * 16), 256, 0, s>>>(b.e0, b.p0, d0.nx, d0.ny, d0.nz, 16);
+        pool_kernel<<<ew_grid(d1.v() * 2), 256, 0, s>>>(b.e0, b.p0, d0.nx, d0.ny, d0.nz, 16);
         MF3D_LAUNCH_CK();
         layer(s, 2, d1, b.p0, b.a2);
         layer(s, 3, d1, b.a2, b.e1);
-        pool_kernel<<<ew_grid(d2.v() * 32), 256, 0, s>>>(b.e1, b.p1, d1.nx, d1.ny, d1.nz, 32);
+        pool_kernel<<<ew_grid(d2.v() * 4), 256, 0, s>>>(b.e1, b.p1, d1.nx, d1.ny, d1.nz, 32);
         MF3D_LAUNCH_CK();
         layer(s, 4, d2, b.p1, b.a4);
         layer(s, 5, d2, b.a4, b.e2);
-        pool_kernel<<<ew_grid(d3.v() * 64), 256, 0, s>>>(b.e2, b.p2, d2.nx, d2.ny, d2.nz, 64);
+        pool_kernel<<<ew_grid(d3.v() * 8), 256, 0, s>>>(b.e2, b.p2, d2.nx, d2.ny, d2.nz, 64);
         MF3D_LAUNCH_CK();
         layer(s, 6, d3, b.p2, b.a6);
         layer(s, 7, d3, b.a6, b.e3);
@@ -442,9 +440,6 @@ class WarmStartNet {
         __nv_bfloat16* g = b.g0;  // gradient being consumed
         __nv_bfloat16* gn = b.g1; // gradient being produced
         auto swap = [&] { std::swap(g, gn); };
-        MF3D_CK(cudaMemsetAsync(b.acc0, 0, d0.v() * 16 * 4, s));
-        MF3D_CK(cudaMemsetAsync(b.acc1, 0, d1.v() * 32 * 4, s));
-        MF3D_CK(cudaMemsetAsync(b.acc2, 0, d2.v() * 64 * 4, s));
         // layer 11 (linear output)
         wg(s, 11, d0, b.d0, b.dout);
         dgrad(s, 11, d0, b.dout, b.d0, gn); // d pre-activation of layer 10
@@ -453,33 +448,21 @@ class WarmStartNet {
         wg(s, 10, d0, b.c0, g);
         dgrad(s, 10, d0, g, nullptr, gn); // d c0 (48 channels)
         swap();
-        upcat_bwd_skip_kernel<<<ew_grid(d0.v() * 16), 256, 0, s>>>(g, b.acc0, d0.v(), 32, 16);
-        MF3D_LAUNCH_CK();
-        upcat_bwd_coarse_kernel<<<ew_grid(d1.v() * 32), 256, 0, s>>>(g, b.accc, d0.nx, d0.ny, d0.nz, 32, 16);
-        MF3D_LAUNCH_CK();
-        mask_to_bf16_kernel<<<ew_grid(d1.v() * 32), 256, 0, s>>>(b.accc, b.d1, gn, d1.v() * 32);
+        upcat_bwd_kernel<<<ew_grid(d1.v() * 6), 256, 0, s>>>(g, b.d1, gn, b.sk0, d0.nx, d0.ny, d0.nz, 32, 16);
         MF3D_LAUNCH_CK();
         swap(); // d pre-activation of layer 9
         // layer 9 on c1 = up(d2) ++ e1
         wg(s, 9, d1, b.c1, g);
         dgrad(s, 9, d1, g, nullptr, gn); // d c1 (96)
         swap();
-        upcat_bwd_skip_kernel<<<ew_grid(d1.v() * 32), 256, 0, s>>>(g, b.acc1, d1.v(), 64, 32);
-        MF3D_LAUNCH_CK();
-        upcat_bwd_coarse_kernel<<<ew_grid(d2.v() * 64), 256, 0, s>>>(g, b.accc, d1.nx, d1.ny, d1.nz, 64, 32);
-        MF3D_LAUNCH_CK();
-        mask_to_bf16_kernel<<<ew_grid(d2.v() * 64), 256, 0, s>>>(b.accc, b.d2, gn, d2.v() * 64);
+        upcat_bwd_kernel<<<ew_grid(d2.v() * 12), 256, 0, s>>>(g, b.d2, gn, b.sk1, d1.nx, d1.ny, d1.nz, 64, 32);
         MF3D_LAUNCH_CK();
         swap(); // layer 8 pre-activation
         // layer 8 on c2 = up(e3) ++ e2
         wg(s, 8, d2, b.c2, g);
         dgrad(s, 8, d2, g, nullptr, gn); // d c2 (128)
         swap();
-        upcat_bwd_skip_kernel<<<ew_grid(d2.v() * 64), 256, 0, s>>>(g, b.acc2, d2.v(), 64, 64);
-        MF3D_LAUNCH_CK();
-        upcat_bwd_coarse_kernel<<<ew_grid(d3.v() * 64), 256, 0, s>>>(g, b.accc, d2.nx, d2.ny, d2.nz, 64, 64);
-        MF3D_LAUNCH_CK();
-        mask_to_bf16_kernel<<<ew_grid(d3.v() * 64), 256, 0, s>>>(b.accc, b.e3, gn, d3.v() * 64);
+        upcat_bwd_kernel<<<ew_grid(d3.v() * 16), 256, 0, s>>>(g, b.e3, gn, b.sk2, d2.nx, d2.ny, d2.nz, 64, 64);
         MF3D_LAUNCH_CK();
         swap(); // layer 7 pre-activation
         // encoder L3
@@ -489,9 +472,7 @@ class WarmStartNet {
         wg(s, 6, d3, b.p2, g);
         dgrad(s, 6, d3, g, nullptr, gn); // d p2
         swap();
-        pool_bwd_kernel<<<ew_grid(d2.v() * 64), 256, 0, s>>>(g, b.acc2, d2.nx, d2.ny, d2.nz, 64);
-        MF3D_LAUNCH_CK();
-        mask_to_bf16_kernel<<<ew_grid(d2.v() * 64), 256, 0, s>>>(b.acc2, b.e2, gn, d2.v() * 64);
+        skip_pool_bwd_kernel<<<ew_grid(d2.v() * 8), 256, 0, s>>>(b.sk2, g, b.e2, gn, d2.nx, d2.ny, d2.nz, 64);
         MF3D_LAUNCH_CK();
         swap(); // layer 5 pre-activation
         // encoder L2
@@ -501,9 +482,7 @@ class WarmStartNet {
         wg(s, 4, d2, b.p1, g);
         dgrad(s, 4, d2, g, nullptr, gn); // d p1
         swap();
-        pool_bwd_kernel<<<ew_grid(d1.v() * 32), 256, 0, s>>>(g, b.acc1, d1.nx, d1.ny, d1.nz, 32);
-        MF3D_LAUNCH_CK();
-        mask_to_bf16_kernel<<<ew_grid(d1.v() * 32), 256, 0, s>>>(b.acc1, b.e1, gn, d1.v() * 32);
+        skip_pool_bwd_kernel<<<ew_grid(d1.v() * 4), 256, 0, s>>>(b.sk1, g, b.e1, gn, d1.nx, d1.ny, d1.nz, 32);
         MF3D_LAUNCH_CK();
         swap(); // layer 3 pre-activation
         // encoder L1
@@ -513,9 +492,7 @@ class WarmStartNet {
         wg(s, 2, d1, b.p0, g);
         dgrad(s, 2, d1, g, nullptr, gn); // d p0
         swap();
-        pool_bwd_kernel<<<ew_grid(d0.v() * 16), 256, 0, s>>>(g, b.acc0, d0.nx, d0.ny, d0.nz, 16);
-        MF3D_LAUNCH_CK();
-        mask_to_bf16_kernel<<<ew_grid(d0.v() * 16), 256, 0, s>>>(b.acc0, b.e0, gn, d0.v() * 16);
+        skip_pool_bwd_kernel<<<ew_grid(d0.v() * 2), 256, 0, s>>>(b.sk0, g, b.e0, gn, d0.nx, d0.ny, d0.nz, 16);
         MF3D_LAUNCH_CK();
         swap(); // layer 1 pre-activation
         // encoder L0
