@@ -1025,7 +1025,7 @@ int mf3d_batch_create(int count, const mf3d_grid* grids, const mf3d_bc* bc, cons
             const std::vector<char> side = EnsembleSolver::choose(count, grids, c.precision);
             for (int r = 0; r < count; ++r) {
                 const bool alone = side[r] != 0;
-                (alone ? solo : hs).emplace_back(new HeadSolver(grids[r], *bc, c, s));
+                (alone ? solo : hs).emplace_back(new HeadSolver(grids[r], *bc, c, s, alone));
                 (alone ? solo_at : batch_at).push_back(r);
             }
             std::unique_ptr<BatchSolverBase> small;

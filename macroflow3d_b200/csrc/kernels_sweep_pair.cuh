@@ -525,7 +525,9 @@ __global__ void __launch_bounds__(SP_NT, (sp_minb<T, TC, TM>()))
                     if constexpr (PROL) {
                         const P2<T> v = take(sx1, f, en[q]);
                         xnO = O ? v.b : v.a;
-                        en[q] = corr(pin[q], pi0 + QS * q, wj, t + 2);
+                        // (an odd plane's parent is that of the plane before: 0.099 -> 0.095 ms in FP32
+                        // at 256^3, 0.190 -> 0.180 in FP64)
+                        if (!(t & 1)) en[q] = corr(pin[q], pi0 + QS * q, wj, t + 2);
                     } else if constexpr (ZERO) {
                         xnO = (T)0;
                     } else {
@@ -733,8 +735,10 @@ __global__ void __launch_bounds__(SP_NT, (sp_minb<T, TC, TM>()))
                     const P2<T> xnext = take(sx1, f, en[q]);
                     if (has2) (void)take(sx1, fx2 + QS * q, en2[q]);
                     if constexpr (PROL) {
-                        en[q] = corr(pin[q], wi[q], wj, t + 2);
-                        if (has2) en2[q] = corr(pin2[q], wi[q], wj2, t + 2);
+                        if (!(t & 1)) {
+                            en[q] = corr(pin[q], wi[q], wj, t + 2);
+                            if (has2) en2[q] = corr(pin2[q], wi[q], wj2, t + 2);
+                        }
                     }
                     const P2<T> b2 = sp_ld2<T>(C + OB + g), cx2p = sp_ldc<T, TC>(Cc + g);
                     const P2<T> cy2p = sp_ldc<T, TC>(Cc + OCYc + f), cyd2 = sp_ldc<T, TC>(Cc + cyd_off[q]);

@@ -645,9 +645,10 @@ template <class T, class TC> class VCycle : public VCycleBase {
     // r64: the FP64 residual (dot products, and the right-hand side when the whole V-cycle is
     // the coarse tail).
     // cp: the cluster kernel's plan for single solves (cp.Lc <= Lt), or cp.Lc = -1
+    // single: false for a realisation that is only solved in a batch (no matrix, no map of the coarsest level)
     VCycle(const std::vector<Geom>& G, int Lt, const CoarsePlan& cp, const mf3d_bc& bc, bool pin, int pre, int post,
            int coarse, const std::vector<LevelOp<double>>& op64, Scratch scr, const T* b0, const double* r64,
-           bool allow_tma)
+           bool allow_tma, bool single)
         : G_(G), Lt_(Lt), cp_(cp), bc_(bc), pin_(pin), pre_(pre), post_(post), coarse_(coarse), op64_(op64),
           scr_(scr), b0_(b0), r64_(r64) {
         const int nl = (int)G.size();
@@ -772,7 +773,7 @@ template <class T, class TC> class VCycle : public VCycleBase {
                     cp_.a.post = post;
                     cp_.a.coarse_iters = coarse;
                     cp_.a.M = nullptr;
-                    if (cp_.a.moff >= 0) {
+                    if (cp_.a.moff >= 0 && single) {
                         const CLevel& C = cp_.a.L[cp_.a.nlev - 1];
                         cmap_.reset(new DevMem((size_t)C.n * 2 * C.hcap * sizeof(double)));
                         bytes_ += cmap_->bytes;
@@ -803,7 +804,7 @@ template <class T, class TC> class VCycle : public VCycleBase {
                 T2.w = tail_w_->as<double>() + woff;
                 woff += 8 * G[l].n;
             }
-            plan_dense(nl);
+            if (single) plan_dense(nl);
             tail_smem_ = (size_t)off * sizeof(double);
             tail_out_.reset(new DevMem(G[Lt].n * sizeof(T)));
             bytes_ += G[Lt].n * sizeof(T);
@@ -1545,7 +1546,8 @@ class HeadSolver {
     friend class EnsembleSolver;
 
   public:
-    HeadSolver(const mf3d_grid& g, const mf3d_bc& bc, const mf3d_solver_config& cfg, cudaStream_t user_stream)
+    HeadSolver(const mf3d_grid& g, const mf3d_bc& bc, const mf3d_solver_config& cfg, cudaStream_t user_stream,
+               bool single = true)
         : grid_(g), bc_(bc), cfg_(cfg) {
         if (g.nx < 2 || g.ny < 2 || g.nz < 2) throw Error(MF3D_E_INVALID, "grid must have at least 2 cells per axis");
         if (!(g.dx > 0)) throw Error(MF3D_E_INVALID, "dx must be positive");
@@ -1636,14 +1638,14 @@ class HeadSolver {
         }
         if (prec == MF3D_PREC_FP64)
             vc_.reset(new VCycle<double, double>(G_, Lt_, cplan_, bc, pin_, cfg.mg_pre_smooth, cfg.mg_post_smooth,
-                                                 cfg.mg_coarse_iters, op64_, scr, r_.as<double>(), r_.as<double>(), tma));
+                                                 cfg.mg_coarse_iters, op64_, scr, r_.as<double>(), r_.as<double>(), tma, single));
         else if (prec == MF3D_PREC_FP32)
             vc_.reset(new VCycle<float, float>(G_, Lt_, cplan_, bc, pin_, cfg.mg_pre_smooth, cfg.mg_post_smooth,
-                                               cfg.mg_coarse_iters, op64_, scr, r32_.as<float>(), r_.as<double>(), tma));
+                                               cfg.mg_coarse_iters, op64_, scr, r32_.as<float>(), r_.as<double>(), tma, single));
         else if (prec == MF3D_PREC_BF16)
             vc_.reset(new VCycle<float, __nv_bfloat16>(G_, Lt_, cplan_, bc, pin_, cfg.mg_pre_smooth, cfg.mg_post_smooth,
                                                        cfg.mg_coarse_iters, op64_, scr, r32_.as<float>(),
-                                                       r_.as<double>(), tma));
+                                                       r_.as<double>(), tma, single));
         else
             throw Error(MF3D_E_INVALID, "unknown precision");
         bytes_ += vc_->bytes();
@@ -1868,14 +1870,14 @@ class HeadSolver {
 
     // mode 0: of x_, into r_; 1: of the head `x`, the norm only (into scratch)
     void launch_residual(cudaStream_t s, int mode, const double* x = nullptr) {
-        const size_t n = G_[0].n;
         double* out = mode == 0 ? r_.as<double>() : Ap_.as<double>();
-        (void)n;
+        if (!x) x = x_.as<double>();
+        float* r32 = mode == 1 ? nullptr : r32_.as<float>();
+        const int ref_is_b = cfg_.conv_norm == MF3D_CONV_B ? 1 : 0;
         const ColLaunch cl = col_launch(G_[0].nx, G_[0].ny, G_[0].nz);
-        residual_kernel<double><<<cl.grid, cl.block, 0, s>>>(
-            op64_[0], x ? x : x_.as<double>(), b_.as<double>(), out, state_.as<PcgState>(), partials_.as<double>(),
-            tickets_.as<unsigned>() + 2, mode, cfg_.conv_norm == MF3D_CONV_B ? 1 : 0,
-            mode == 1 ? nullptr : r32_.as<float>(), cond_, 0, cl.zchunk);
+        residual_kernel<double><<<cl.grid, cl.block, 0, s>>>(op64_[0], x, b_.as<double>(), out, state_.as<PcgState>(),
+                                                             partials_.as<double>(), tickets_.as<unsigned>() + 2, mode,
+                                                             ref_is_b, r32, cond_, 0, cl.zchunk);
         MF3D_LAUNCH_CK();
     }
 

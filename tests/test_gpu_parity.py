@@ -650,3 +650,33 @@ def test_velocity_and_diagnostics_edges_vs_numpy(mf3d, shape, per):
         scale = max(np.abs(o).max(), np.abs(u).max() / dx)
         assert np.abs(_np(a) - o).max() <= 1e-13 * max(scale, scale ** 2)
         assert np.allclose(s, (o.min(), o.max(), o.mean()), rtol=1e-11, atol=1e-11 * max(scale, scale ** 2))
+
+
+# the coarse end by its ways: bricks above a matrix with ragged bricks; the matrix alone from the coarsest level
+# of more than 1024 cells; the cluster with a cell of each colour per thread (6175 cells); an odd periodic
+# count on the coarsest level; a hierarchy that is one matrix
+@pytest.mark.parametrize("shape,levels,per", [((24, 40, 56), 4, False), ((20, 24, 28), 2, False),
+                                              ((26, 38, 50), 2, False), ((48, 96, 80), 5, True),
+                                              ((12, 20, 36), 3, True), ((8, 10, 12), 2, False)])
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_coarse_end_ways_match_one_cta_tail(mf3d, monkeypatch, shape, levels, per, prec):
+    """Against the same V-cycle with sweeps down to the one-CTA tail: the same arithmetic in another order, so
+    equal to rounding (1e-12 in FP64, 1e-5 where FP32 levels are swept by another kernel)."""
+    M = mf3d
+    rng = np.random.default_rng(sum(shape) + levels)
+    K, r = np.exp(rng.normal(size=shape)), rng.normal(size=shape)
+    g = M.Grid3D(shape[2], shape[1], shape[0], 0.5)
+    bc = _bcs(M, [D, D] + ([P, P, P, P] if per else [N, N, N, N]), [1.0, 0.0, 0, 0, 0, 0])
+    cfg = M.HeadSolveConfig(mg_levels=levels, precision={"fp64": M.PREC_FP64, "fp32": M.PREC_FP32}[prec])
+    z = []
+    for tail in (False, True):
+        if tail:
+            monkeypatch.setenv("MF3D_NO_CLUSTER_TAIL", "1")
+        s = M.HeadSolver(g, bc, cfg)
+        s.set_K(_t(K))
+        zz = _t(np.zeros(shape))
+        s.vcycle(_t(r), zz)
+        z.append(_np(zz))
+        s.close()
+    monkeypatch.delenv("MF3D_NO_CLUSTER_TAIL", raising=False)
+    assert _rel(z[0], z[1]) < (1e-12 if prec == "fp64" else 1e-5)
