@@ -248,7 +248,8 @@ int mf3d_batch_solve(mf3d_batch* b, double* const* h_dev, const double* const* x
 /* Autotuner (no counterpart in the reference): for every sweep position of the batched
  * V-cycle, times the candidate work-item shapes (z chunks per tile 1, 2, 4, 8; staged or L1
  * sweep) on this batch, `reps` launches each, and keeps the fastest.  Fills up to `cap`
- * records and sets *count.  The solver state is scratch afterwards (the next solve rebuilds it). */
+ * records and sets *count (0 when every realisation is solved side by side by its own single-solve
+ * launches, which have no shapes to tune).  The solver state is scratch afterwards (the next solve rebuilds it). */
 int mf3d_batch_autotune(mf3d_batch* b, int reps, mf3d_batch_tuning* out, int cap, int* count);
 
 /* ---- learned warm start (no counterpart in the reference, whose initial guess is the

@@ -155,8 +155,9 @@ class HeadSolver:
 
     @property
     def coarse_info(self) -> tuple:
-        """(first level of the coarse-end kernel of a single solve, CTAs of its thread-block
-        cluster; 0 when one CTA runs the levels of at most 4096 cells)."""
+        """(first level of the FP64 coarse end of a single solve, CTAs of the thread-block cluster
+        that is planned for it; 0 when one CTA would run the levels of at most 4096 cells).  Bricks
+        and a matrix serve the coarse end instead where they apply."""
         first, ctas = C.c_int(0), C.c_int(0)
         check(lib().mf3d_head_solver_coarse_info(self._h, C.byref(first), C.byref(ctas)))
         return first.value, ctas.value
@@ -204,8 +205,8 @@ class HeadSolver:
 class BatchSolver:
     """Independent head solves of several realisations, each on its own grid, solved together
     (the realisation loop of run_ensemble, src/runtime/ensemble/EnsembleRunner.cu:259-317,
-    without the loop): batched launches, one CUDA graph for the whole PCG loop of all
-    realisations, and a per-realisation stopping test."""
+    without the loop): the larger realisations by their own graphs on four streams, the smaller
+    ones by batched launches in one CUDA graph with a per-realisation stopping test."""
 
     def __init__(self, grids: Sequence[Grid3D], bc: BCSpec, cfg: Optional[HeadSolveConfig] = None,
                  stream=None):
@@ -258,7 +259,8 @@ class BatchSolver:
 
     def autotune(self, reps: int = 3):
         """Times the candidate work-item shapes of every sweep position of the batched V-cycle
-        and keeps the fastest; returns one dict per sweep position."""
+        and keeps the fastest; returns one dict per sweep position (none when every realisation is
+        solved side by side by its own single-solve launches: at most four small grids, or none)."""
         cap = 256
         arr = (_lib.BatchTuning * cap)()
         cnt = C.c_int(0)

@@ -847,6 +847,8 @@ class EnsembleSolver : public BatchSolverBase {
                    cudaStream_t s, cudaStream_t own)
         : solo_(std::move(solo)), solo_at_(std::move(solo_at)), batch_(std::move(batch)),
           batch_at_(std::move(batch_at)), cfg_(cfg), s_(s), own_stream_(own) {
+        for (const auto& h : solo_) // (as for the batch)
+            if (h->Lt_ < 1) throw Error(MF3D_E_INVALID, "batched solve: every grid needs a level above the coarse tail");
         // the largest first, each to the stream with the fewest cells so far
         order_.resize(solo_.size());
         for (size_t i = 0; i < order_.size(); ++i) order_[i] = (int)i;

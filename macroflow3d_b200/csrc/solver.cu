@@ -44,6 +44,8 @@ static thread_local std::string g_err;
 static constexpr size_t kTailSmemMax = 200 * 1024;
 // ... and of one CTA of the cluster kernel (x, b and the weights of its slabs)
 static constexpr size_t kCoarseSmemMax = 224 * 1024;
+// ... and of one unit vector's cycle for the matrix of the coarsest levels
+static constexpr size_t kDenseSmemMax = 100 * 1024;
 
 // Device-time limit of one solve by default: the PCG loop stops with status 3 after this long
 // (mf3d_head_solver_set_time_budget changes it per solver).
@@ -773,7 +775,7 @@ template <class T, class TC> class VCycle : public VCycleBase {
                     cp_.a.post = post;
                     cp_.a.coarse_iters = coarse;
                     cp_.a.M = nullptr;
-                    if (cp_.a.moff >= 0 && single) {
+                    if (cp_.a.moff >= 0 && single && dense_level(nl) < 0) {
                         const CLevel& C = cp_.a.L[cp_.a.nlev - 1];
                         cmap_.reset(new DevMem((size_t)C.n * 2 * C.hcap * sizeof(double)));
                         bytes_ += cmap_->bytes;
@@ -862,7 +864,8 @@ template <class T, class TC> class VCycle : public VCycleBase {
             wo += 8 * G_[l].n;
         }
         if (dense_) { // the cycle on the levels from D_ on as a matrix, one column per cell
-            MF3D_CK(cudaMemsetAsync(dense_->p, 0, dense_->bytes, s));
+            if (dense_ld_ > dtail_.L[0].n) // (the padding column; the others are written)
+                MF3D_CK(cudaMemsetAsync(dense_->p, 0, (size_t)dtail_.L[0].n * dense_ld_ * sizeof(double), s));
             dense_map_kernel<<<dtail_.L[0].n, DN_NT, dtail_smem_, s>>>(dtail_, dense_ld_, dense_->as<double>());
             MF3D_LAUNCH_CK();
         } else if (cmap_) { // the coarsest level's sweeps as a matrix, one column per cell
@@ -1076,13 +1079,20 @@ template <class T, class TC> class VCycle : public VCycleBase {
     // at most DN_MAX_LAST) run their legs in bricks, and the cycle from D_ on is a matrix product.  Where
     // neither size fits, or other sweep counts need a level of legs, the cluster kernel or the one-CTA tail
     // serves.
-    void plan_dense(int nl) {
+    int dense_level(int nl) const { // D_, or -1
         const int Ls = cp_.Lc >= 0 ? cp_.Lc : Lt_;
-        if (std::getenv("MF3D_NO_CLUSTER_TAIL")) return;
+        if (std::getenv("MF3D_NO_CLUSTER_TAIL")) return -1;
         int D = Ls;
         while (D < nl && G_[D].n > (size_t)DN_MAX) ++D;
         if (D == nl && G_[nl - 1].n <= (size_t)DN_MAX_LAST) D = nl - 1;
-        if (D == nl || D < Lt_ || (D > Ls && !(pre_ == 2 && post_ == 2))) return;
+        if (D == nl || D < Lt_ || (D > Ls && !(pre_ == 2 && post_ == 2))) return -1;
+        size_t smem = 0; // of the cycle that builds the matrix
+        for (int l = D; l < nl; ++l) smem += 8 * ((size_t)(G_[l].nx + 2) * (G_[l].ny + 2) * (G_[l].nz + 2) + G_[l].n);
+        return smem > kDenseSmemMax ? -1 : D;
+    }
+    void plan_dense(int nl) {
+        const int Ls = cp_.Lc >= 0 ? cp_.Lc : Lt_, D = dense_level(nl);
+        if (D < 0) return;
         dtail_ = tail_;
         dtail_.nlev = nl - D;
         int off = 0;
@@ -1095,19 +1105,17 @@ template <class T, class TC> class VCycle : public VCycleBase {
             off += L.n;
         }
         dtail_smem_ = (size_t)off * sizeof(double);
-        if (dtail_smem_ > 100 * 1024) return;
-        MF3D_CK(cudaFuncSetAttribute(dense_map_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        MF3D_CK(cudaFuncSetAttribute(dense_map_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmemMax));
         const int n = (int)G_[D].n;
         dense_ld_ = n + (n & 1);
-        dense_.reset(new DevMem((size_t)n * dense_ld_ * sizeof(double)));
-        bytes_ += dense_->bytes;
         D_ = D;
         size_t total = 0; // FP64 vectors: b, x (down leg) and x (up leg) of the levels Ls .. D
         c64_.resize(nl);
         for (int l = Ls; l <= D; ++l) total += 3 * G_[l].n;
-        dvec_.reset(new DevMem(total * sizeof(double)));
-        bytes_ += dvec_->bytes;
-        double* p = dvec_->as<double>();
+        const size_t mat = (size_t)n * dense_ld_;
+        dense_.reset(new DevMem((mat + total) * sizeof(double)));
+        bytes_ += dense_->bytes;
+        double* p = dense_->as<double>() + mat;
         for (int l = Ls; l <= D; ++l) {
             c64_[l] = {p, p + G_[l].n, p + 2 * G_[l].n};
             p += 3 * G_[l].n;
@@ -1507,7 +1515,7 @@ template <class T, class TC> class VCycle : public VCycleBase {
     struct Coarse64 {
         double *b = nullptr, *x = nullptr, *y = nullptr;
     };
-    std::unique_ptr<DevMem> dense_, dvec_; // the matrix of level D_; FP64 vectors of the levels above it
+    std::unique_ptr<DevMem> dense_; // the matrix of level D_, then the FP64 vectors of the levels Ls .. D_
     std::vector<Coarse64> c64_;
     Tail2Args dtail_{};
     int D_ = 0, dense_ld_ = 0;

@@ -214,6 +214,14 @@ def test_nonfinite_realisation_does_not_stop_the_others(mf3d):
     b.close()
 
 
+def test_grids_without_a_level_above_the_tail_are_refused(mf3d):
+    """A grid that is all coarse tail is refused, batched or side by side."""
+    M = mf3d
+    for count in (1, 6):
+        with pytest.raises(M.Mf3dError, match="above the coarse tail"):
+            M.BatchSolver([M.Grid3D(8, 8, 8)] * count, M.BCSpec.darcy_x(), _cfg(M, M.PREC_FP32))
+
+
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_mixed_sizes_keep_their_places(mf3d, prec):
     """Realisations large enough to be solved side by side among seven small ones that are batched:
