@@ -163,6 +163,7 @@ __device__ __forceinline__ bool grid_sums(const double (&v)[NV], double* partial
         for (int q = 0; q < NV; ++q) out[q] = x[q];
         *ticket = 0u;
     }
+    __syncthreads(); // (a block that walks on to another reduction writes red again; only the last block pays)
     return tid == 0;
 }
 

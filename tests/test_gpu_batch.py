@@ -214,6 +214,43 @@ def test_nonfinite_realisation_does_not_stop_the_others(mf3d):
     b.close()
 
 
+def test_reductions_of_successive_blocks_do_not_mix(mf3d):
+    """Ninety-six small realisations: about four thousand virtual blocks of the r update and of the residual on
+    at most eight CTAs a multiprocessor, so every CTA runs several blocks and the last block of one
+    realisation's reduction is followed by a block of another.  Each solve must repeat the first one's counts,
+    residual norms and heads to the last bit (the reductions are deterministic), and equal realisations must
+    agree with each other: their blocks are cut alike and their sums ordered alike."""
+    import torch
+    M = mf3d
+    base = [M.Grid3D(32, 32, 32, 1.0), M.Grid3D(48, 40, 24, 1.0), M.Grid3D(32, 64, 40, 1.0)]
+    Kb = _fields(M, base, seed=800)
+    grids, Ks = base * 32, Kb * 32
+    b, first, _ = _batch(M, grids, M.BCSpec.darcy_x(), _cfg(M, M.PREC_FP64, cg_max_iter=30), Ks)
+    assert b.autotune(1), "the realisations are not batched"
+    hs = [torch.empty_like(K) for K in Ks]
+    b.solve(hs)  # (with the tuned sweeps, repeated below)
+    tuned = None
+    for _ in range(4):
+        res = b.solve(hs)
+        torch.cuda.synchronize()
+        now = [(r.num_iterations, r.initial_residual, r.final_residual, r.true_rel_residual, r.b_norm) for r in res]
+        heads = [h.cpu().numpy() for h in hs]
+        if tuned is not None:
+            assert now == tuned[0]
+            assert all(np.array_equal(x, y) for x, y in zip(heads, tuned[1]))
+        tuned = (now, heads)
+        for r in range(3, len(grids)):
+            assert now[r] == now[r % 3] and np.array_equal(heads[r], heads[r % 3]), r
+    for r in range(3, len(grids)):
+        assert first[r][1].final_residual == first[r % 3][1].final_residual, r
+        assert np.array_equal(first[r][0], first[r % 3][0]), r
+    ref = _single(M, base, M.BCSpec.darcy_x(), _cfg(M, M.PREC_FP64, cg_max_iter=30), Kb)
+    for (hr, rr), (hb, rb) in zip(ref, first):
+        assert rb.converged and abs(rb.num_iterations - rr.num_iterations) <= ITER_SLACK["fp64"]
+        assert _rel(hb, hr) < HEAD_TOL
+    b.close()
+
+
 def test_grids_without_a_level_above_the_tail_are_refused(mf3d):
     """A grid that is all coarse tail is refused, batched or side by side."""
     M = mf3d
