@@ -57,6 +57,8 @@ class BatchSolverBase {
     virtual std::vector<mf3d_batch_tuning> autotune(int reps) = 0;
     virtual long long device_bytes() const = 0;
     virtual int count() const = 0;
+    virtual double* x_of(int r) const = 0; // realisation r's own head vector
+    virtual size_t cells_of(int r) const = 0;
 };
 
 // host-side layout of a small device table: appends arrays at 256-byte boundaries
@@ -289,6 +291,8 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
     }
 
     int count() const override { return (int)hs_.size(); }
+    double* x_of(int r) const override { return hs_[r]->x_.template as<double>(); }
+    size_t cells_of(int r) const override { return hs_[r]->G_[0].n; }
 
     long long device_bytes() const override {
         long long b = 0;
@@ -849,6 +853,9 @@ class EnsembleSolver : public BatchSolverBase {
           batch_at_(std::move(batch_at)), cfg_(cfg), s_(s), own_stream_(own) {
         for (const auto& h : solo_) // (as for the batch)
             if (h->Lt_ < 1) throw Error(MF3D_E_INVALID, "batched solve: every grid needs a level above the coarse tail");
+        place_.resize(count());
+        for (size_t i = 0; i < solo_at_.size(); ++i) place_[solo_at_[i]] = (int)i;
+        for (size_t i = 0; i < batch_at_.size(); ++i) place_[batch_at_[i]] = -1 - (int)i;
         // the largest first, each to the stream with the fewest cells so far
         order_.resize(solo_.size());
         for (size_t i = 0; i < order_.size(); ++i) order_[i] = (int)i;
@@ -887,6 +894,14 @@ class EnsembleSolver : public BatchSolverBase {
     }
 
     int count() const override { return (int)(solo_.size() + batch_at_.size()); }
+    double* x_of(int r) const override {
+        const int i = place_[r];
+        return i >= 0 ? solo_[i]->x_.as<double>() : batch_->x_of(-1 - i);
+    }
+    size_t cells_of(int r) const override {
+        const int i = place_[r];
+        return i >= 0 ? solo_[i]->G_[0].n : batch_->cells_of(-1 - i);
+    }
     long long device_bytes() const override {
         long long b = batch_ ? batch_->device_bytes() : 0;
         for (const auto& h : solo_) b += h->device_bytes();
@@ -913,7 +928,9 @@ class EnsembleSolver : public BatchSolverBase {
         std::vector<mf3d_solve_result> part(batch_at_.size());
         const long long l0 = g_launches;
         MF3D_CK(cudaEventRecord(ev0_, s_));
-        auto x0_of = [&](int r) { return x0 ? x0[r] : nullptr; };
+        std::vector<const double*> guess;
+        if (x0) guess = read_early(h, x0);
+        auto x0_of = [&](int r) { return x0 ? guess[r] : nullptr; };
         if (cfg_.use_graph) {
             on_lanes([&](int i, cudaStream_t s) { solo_[i]->enqueue(h[solo_at_[i]], x0_of(solo_at_[i]), s); });
         } else { // (host-driven loops wait: one solve after the other)
@@ -956,6 +973,39 @@ class EnsembleSolver : public BatchSolverBase {
         cudaStream_t s = nullptr;
         cudaEvent_t done = nullptr;
     };
+    // Every guess is read before any head is written, as in one batch: a guess that lies in an array where
+    // another realisation solved side by side puts its head (heads handed on between realisations, arrays used
+    // in turn) goes to that solver's own vector first.  Returns where each guess is to be read.
+    std::vector<const double*> read_early(double* const* h, const double* const* x0) {
+        struct Range {
+            const double *lo, *hi;
+            int r;
+        };
+        const int R = count();
+        std::vector<const double*> from(x0, x0 + R);
+        std::vector<Range> out; // the heads written side by side, by address
+        for (int r : solo_at_) out.push_back({h[r], h[r] + cells_of(r), r});
+        std::sort(out.begin(), out.end(), [](const Range& a, const Range& b) { return a.lo < b.lo; });
+        size_t longest = 0;
+        for (const Range& w : out) longest = std::max(longest, (size_t)(w.hi - w.lo));
+        for (int r = 0; r < R; ++r) {
+            if (!x0[r]) continue;
+            const double *lo = x0[r], *hi = lo + cells_of(r);
+            // heads that begin before the guess ends and not more than the longest one before it begins
+            auto it = std::lower_bound(out.begin(), out.end(), hi, [](const Range& w, const double* p) { return w.lo < p; });
+            bool other = false;
+            while (it != out.begin() && !other) {
+                --it;
+                other = it->hi > lo && it->r != r;
+                if (it->lo + longest <= lo) break;
+            }
+            if (!other) continue;
+            double* own = x_of(r);
+            MF3D_CK(cudaMemcpyAsync(own, x0[r], cells_of(r) * sizeof(double), cudaMemcpyDeviceToDevice, s_));
+            from[r] = own;
+        }
+        return from;
+    }
     // f(i, stream) for every solo realisation, on the lanes' streams between what s_ held before and what
     // comes after
     template <class F> void on_lanes(F&& f) {
@@ -986,6 +1036,7 @@ class EnsembleSolver : public BatchSolverBase {
     std::vector<int> batch_at_;
     mf3d_solver_config cfg_;
     cudaStream_t s_ = nullptr, own_stream_ = nullptr;
+    std::vector<int> place_; // of a realisation: its index in solo_, or -1 - its index in batch_
     std::vector<int> order_, lane_of_;
     std::vector<Lane> lanes_;
     cudaEvent_t fork_ = nullptr, ev0_ = nullptr, ev1_ = nullptr;

@@ -1761,8 +1761,8 @@ class HeadSolver {
         const long long l0 = g_launches;
         body_runs_ = 0;
         MF3D_CK(cudaEventRecord(ev0_, s));
-        if (x0) MF3D_CK(cudaMemcpyAsync(x_.p, x0, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        else launch_guess(s, G_[0], bc_, x_.as<double>());
+        if (x0 && x0 != x_.p) MF3D_CK(cudaMemcpyAsync(x_.p, x0, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        else if (!x0) launch_guess(s, G_[0], bc_, x_.as<double>());
         MF3D_CK(cudaMemsetAsync(tickets_.p, 0, tickets_.bytes, s));
         const bool mg = cfg_.solver == MF3D_SOLVER_MG, cg = cfg_.solver == MF3D_SOLVER_CG;
         pcg_init_kernel<<<1, 1, 0, s>>>(state_.as<PcgState>(), mg ? cfg_.mg_max_cycles : cfg_.cg_max_iter,

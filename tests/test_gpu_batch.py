@@ -214,6 +214,54 @@ def test_nonfinite_realisation_does_not_stop_the_others(mf3d):
     b.close()
 
 
+def test_guesses_in_other_realisations_heads(mf3d):
+    """Warm starts that lie in the arrays of other realisations' heads (arrays used in turn, a guess inside a larger
+    head): every guess is read before any head is written, so each realisation starts from its converged head
+    and is done after one step at most.  Six realisations are solved side by side, two on some streams, and
+    five as one batch."""
+    import torch
+    M = mf3d
+    grids = [M.Grid3D(64, 48, 80, 1.0)] * 6 + [M.Grid3D(32, 32, 32, 1.0)] * 5
+    bc = M.BCSpec.darcy_x()
+    cfg = _cfg(M, M.PREC_FP64)
+    Ks = _fields(M, grids, seed=900)
+    b, got, _ = _batch(M, grids, bc, cfg, Ks)
+    assert b.autotune(1), "no realisation is batched"
+    heads = [torch.from_numpy(h).cuda() for h, _ in got]
+    hs = [torch.empty_like(K) for K in Ks]
+    x0s = [None] * len(grids)
+    for r in range(6):  # the head of r is in the array that realisation r + 1 writes
+        x0s[r] = hs[(r + 1) % 6]
+        x0s[r].copy_(heads[r])
+    n = 32 ** 3
+    for r in range(6, 9):  # a batched realisation's guess inside a larger array, from an odd cell on
+        hs[r - 6].view(-1)[101:101 + n].copy_(heads[r].view(-1))
+        x0s[r] = hs[r - 6].view(-1)[101:101 + n]
+        x0s[(r - 7) % 6] = None  # (the guess that was there)
+    x0s[9], x0s[10] = hs[10], hs[9]  # two batched ones crosswise
+    x0s[9].copy_(heads[9])
+    x0s[10].copy_(heads[10])
+    assert sum(x is not None for x in x0s[:6]) == 3
+    res = b.solve(hs, x0s)
+    torch.cuda.synchronize()
+    for r, one in enumerate(res):
+        assert one.converged
+        if x0s[r] is not None:
+            assert one.num_iterations <= 1, r
+        assert _rel(hs[r].cpu().numpy(), got[r][0]) < HEAD_TOL, r
+    # all six crosswise, and a realisation's guess in its own head's array
+    for r in range(6):
+        x0s[r] = hs[(r + 1) % 6]
+        x0s[r].copy_(heads[r])
+    for r in range(6, 11):
+        x0s[r] = hs[r]
+    res = b.solve(hs, x0s)
+    torch.cuda.synchronize()
+    for r, one in enumerate(res):
+        assert one.num_iterations <= 1 and _rel(hs[r].cpu().numpy(), got[r][0]) < HEAD_TOL, r
+    b.close()
+
+
 def test_reductions_of_successive_blocks_do_not_mix(mf3d):
     """Ninety-six small realisations: about four thousand virtual blocks of the r update and of the residual on
     at most eight CTAs a multiprocessor, so every CTA runs several blocks and the last block of one
