@@ -921,10 +921,11 @@ class EnsembleSolver : public BatchSolverBase {
     }
 
     void solve(double* const* h, const double* const* x0, mf3d_solve_result* res) override {
-        for (size_t i = 0; i < solo_.size(); ++i) {
-            if (!solo_[i]->have_K_) throw Error(MF3D_E_STATE, "set_K must be called before solve");
-            if (!h[solo_at_[i]]) throw Error(MF3D_E_INVALID, "h is null");
-        }
+        // (all of them, the batched ones too, before anything starts)
+        for (const auto& one : solo_)
+            if (!one->have_K_) throw Error(MF3D_E_STATE, "set_K must be called before solve");
+        for (int r = 0; r < count(); ++r)
+            if (!h[r]) throw Error(MF3D_E_INVALID, "h is null");
         std::vector<mf3d_solve_result> part(batch_at_.size());
         const long long l0 = g_launches;
         MF3D_CK(cudaEventRecord(ev0_, s_));

@@ -262,6 +262,30 @@ def test_guesses_in_other_realisations_heads(mf3d):
     b.close()
 
 
+def test_missing_head_of_a_batched_realisation_refuses_the_call(mf3d):
+    """A null head among the batched realisations is refused before a solve side by side starts: no other head
+    is touched, and the next call works."""
+    import torch
+    M = mf3d
+    from macroflow3d_b200 import _lib
+    grids = [M.Grid3D(64, 48, 80, 1.0)] * 2 + [M.Grid3D(32, 32, 32, 1.0)] * 5
+    Ks = _fields(M, grids, seed=950)
+    b = M.BatchSolver(grids, M.BCSpec.darcy_x(), _cfg(M, M.PREC_FP64))
+    b.set_K(Ks)
+    hs = [torch.full_like(K, float("nan")) for K in Ks]
+    torch.cuda.synchronize()
+    ptrs = b._ptrs(hs, "h")
+    ptrs[4] = None
+    res = (_lib.SolveResult * len(grids))()
+    assert _lib.lib().mf3d_batch_solve(b._h, ptrs, None, res) == _lib.MF3D_E_INVALID
+    torch.cuda.synchronize()
+    assert all(bool(torch.isnan(h).all()) for h in hs)
+    assert all(r.converged for r in b.solve(hs))
+    torch.cuda.synchronize()
+    assert all(bool(torch.isfinite(h).all()) for h in hs)
+    b.close()
+
+
 def test_reductions_of_successive_blocks_do_not_mix(mf3d):
     """Ninety-six small realisations: about four thousand virtual blocks of the r update and of the residual on
     at most eight CTAs a multiprocessor, so every CTA runs several blocks and the last block of one
