@@ -245,6 +245,9 @@ int mf3d_batch_set_K(mf3d_batch* b, const double* const* K_dev);
  * results[r] as mf3d_head_solve's; device_ms and kernel_launches are the whole batch's. */
 int mf3d_batch_solve(mf3d_batch* b, double* const* h_dev, const double* const* x0_dev,
                      mf3d_solve_result* results);
+/* Diagnostics, no counterpart in the reference: sets the error flag of one realisation as a pipeline
+ * wait that gave up in its smoother would, between solves (the next solve reports it and clears it). */
+int mf3d_diag_raise_pipeline_flag(mf3d_batch* b, int realisation);
 /* Autotuner (no counterpart in the reference): for every sweep position of the batched
  * V-cycle, times the candidate work-item shapes (z chunks per tile 1, 2, 4, 8; staged or L1
  * sweep) on this batch, `reps` launches each, and keeps the fastest.  Fills up to `cap`

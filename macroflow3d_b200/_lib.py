@@ -92,6 +92,7 @@ SIGNATURES = {
     "mf3d_velocity_mass_balance": ([_G, _B, _P, _P, _P, _P, _P, C.POINTER(C.c_double), _P], C.c_int),
     "mf3d_velocity_mass_balance_noalloc": ([_G, _B, _P, _P, _P, _P, _P, C.POINTER(C.c_double), _P], C.c_int),
     "mf3d_head_solver_set_time_budget": ([_P, C.c_double], C.c_int),
+    "mf3d_diag_raise_pipeline_flag": ([C.c_void_p, C.c_int], C.c_int),
     "mf3d_diag_bounded_wait": ([C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int)], C.c_int),
     "mf3d_velocity_diagnostics": ([_G, C.c_int, _P, _P, _P, _P, _P, _P, C.POINTER(C.c_double), _P], C.c_int),
     "mf3d_apply_A": ([_G, _B, C.c_int, _P, _P, _P, _P], C.c_int),

@@ -19,6 +19,7 @@
 // staged and the L1 sweep) is picked per sweep position by an autotuner that times the
 // candidates on the batch itself.
 #pragma once
+#include "in_turn.hpp"
 #include "kernels_batch.cuh"
 
 namespace mf3d {
@@ -59,6 +60,7 @@ class BatchSolverBase {
     virtual int count() const = 0;
     virtual double* x_of(int r) const = 0; // realisation r's own head vector
     virtual size_t cells_of(int r) const = 0;
+    virtual void raise_flag(int r) = 0; // as a pipeline of realisation r that gave up does
 };
 
 // host-side layout of a small device table: appends arrays at 256-byte boundaries
@@ -293,6 +295,7 @@ template <class T, class TC> class BatchSolverT : public BatchSolverBase {
     int count() const override { return (int)hs_.size(); }
     double* x_of(int r) const override { return hs_[r]->x_.template as<double>(); }
     size_t cells_of(int r) const override { return hs_[r]->G_[0].n; }
+    void raise_flag(int r) override { hs_[r]->raise_flag(); }
 
     long long device_bytes() const override {
         long long b = 0;
@@ -902,6 +905,11 @@ class EnsembleSolver : public BatchSolverBase {
         const int i = place_[r];
         return i >= 0 ? solo_[i]->G_[0].n : batch_->cells_of(-1 - i);
     }
+    void raise_flag(int r) override {
+        const int i = place_[r];
+        if (i >= 0) solo_[i]->raise_flag();
+        else batch_->raise_flag(-1 - i);
+    }
     long long device_bytes() const override {
         long long b = batch_ ? batch_->device_bytes() : 0;
         for (const auto& h : solo_) b += h->device_bytes();
@@ -938,24 +946,31 @@ class EnsembleSolver : public BatchSolverBase {
             for (size_t i = 0; i < solo_.size(); ++i) solo_[i]->enqueue(h[solo_at_[i]], x0_of(solo_at_[i]), s_);
         }
         MF3D_CK(cudaEventRecord(ev1_, s_));
-        if (batch_) {
-            std::vector<double*> hb;
-            std::vector<const double*> xb;
-            for (int r : batch_at_) {
-                hb.push_back(h[r]);
-                xb.push_back(x0_of(r));
-            }
-            batch_->solve(hb.data(), xb.data(), part.data());
-        }
-        MF3D_CK(cudaStreamSynchronize(s_));
-        float ms = 0.f;
-        MF3D_CK(cudaEventElapsedTime(&ms, ev0_, ev1_));
-        long long launches = g_launches - l0;
         std::vector<mf3d_solve_result> own(solo_.size());
-        for (size_t i = 0; i < solo_.size(); ++i) {
-            solo_[i]->finish(&own[i]);
-            launches += own[i].kernel_launches - solo_[i]->launches_;
-        }
+        float ms = 0.f;
+        long long launches = 0;
+        // a realisation whose pipeline gave up ends the call, but only after every realisation's flag has
+        // been read and cleared: one left set would end the next call
+        each_then_throw(2 + solo_.size(), [&](size_t step) {
+            if (step == 0) {
+                if (!batch_) return;
+                std::vector<double*> hb;
+                std::vector<const double*> xb;
+                for (int r : batch_at_) {
+                    hb.push_back(h[r]);
+                    xb.push_back(x0_of(r));
+                }
+                batch_->solve(hb.data(), xb.data(), part.data());
+            } else if (step == 1) {
+                MF3D_CK(cudaStreamSynchronize(s_));
+                MF3D_CK(cudaEventElapsedTime(&ms, ev0_, ev1_));
+                launches = g_launches - l0;
+            } else {
+                const size_t i = step - 2;
+                solo_[i]->finish(&own[i]);
+                launches += own[i].kernel_launches - solo_[i]->launches_;
+            }
+        });
         if (!part.empty()) {
             ms += part[0].device_ms;
             launches += part[0].kernel_launches;
@@ -1128,6 +1143,14 @@ int mf3d_batch_solve(mf3d_batch* b, double* const* h, const double* const* x0, m
         need(b, "batch");
         need(h, "h");
         b->impl->solve(h, x0, res);
+    });
+}
+
+int mf3d_diag_raise_pipeline_flag(mf3d_batch* b, int realisation) {
+    return guard([&] {
+        need(b, "batch");
+        if (realisation < 0 || realisation >= b->impl->count()) throw Error(MF3D_E_INVALID, "no such realisation");
+        b->impl->raise_flag(realisation);
     });
 }
 

@@ -1746,6 +1746,12 @@ class HeadSolver {
         }
     }
 
+    void raise_flag() {
+        const int one = 1;
+        MF3D_CK(cudaMemcpy(err_.p, &one, sizeof(int), cudaMemcpyHostToDevice));
+        MF3D_CK(cudaDeviceSynchronize());
+    }
+
     void solve(double* h, const double* x0, mf3d_solve_result* res) {
         if (!have_K_) throw Error(MF3D_E_STATE, "set_K must be called before solve");
         if (!h) throw Error(MF3D_E_INVALID, "h is null");

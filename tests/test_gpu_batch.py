@@ -286,6 +286,29 @@ def test_missing_head_of_a_batched_realisation_refuses_the_call(mf3d):
     b.close()
 
 
+def test_flags_of_several_realisations_end_one_call_only(mf3d):
+    """Pipeline flags of two realisations solved side by side and of two batched ones: the call that meets them
+    fails, and the next one has none left."""
+    import torch
+    M = mf3d
+    from macroflow3d_b200 import _lib
+    grids = [M.Grid3D(64, 48, 80, 1.0)] * 3 + [M.Grid3D(32, 32, 32, 1.0)] * 5
+    Ks = _fields(M, grids, seed=970)
+    b, got, _ = _batch(M, grids, M.BCSpec.darcy_x(), _cfg(M, M.PREC_FP64), Ks)
+    hs = [torch.empty_like(K) for K in Ks]
+    for which in ([0, 2], [1, 4, 6], [3, 7], [0, 1, 2, 3, 4, 5, 6, 7]):
+        for r in which:
+            M.check(_lib.lib().mf3d_diag_raise_pipeline_flag(b._h, r))
+        with pytest.raises(M.Mf3dError, match="wait timed out"):
+            b.solve(hs)
+        res = b.solve(hs)
+        torch.cuda.synchronize()
+        for h, one, (hg, rg) in zip(hs, res, got):
+            assert one.num_iterations == rg.num_iterations and np.array_equal(h.cpu().numpy(), hg)
+    assert _lib.lib().mf3d_diag_raise_pipeline_flag(b._h, 8) == _lib.MF3D_E_INVALID
+    b.close()
+
+
 def test_reductions_of_successive_blocks_do_not_mix(mf3d):
     """Ninety-six small realisations: about four thousand virtual blocks of the r update and of the residual on
     at most eight CTAs a multiprocessor, so every CTA runs several blocks and the last block of one
