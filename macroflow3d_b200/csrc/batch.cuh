@@ -1023,16 +1023,23 @@ class EnsembleSolver : public BatchSolverBase {
         return from;
     }
     // f(i, stream) for every solo realisation, on the lanes' streams between what s_ held before and what
-    // comes after
+    // comes after.  When f throws, what has been started is still joined, and waited for: the caller may free
+    // its arrays once the error is back.
     template <class F> void on_lanes(F&& f) {
         if (solo_.empty()) return;
         MF3D_CK(cudaEventRecord(fork_, s_));
-        for (Lane& l : lanes_) MF3D_CK(cudaStreamWaitEvent(l.s, fork_, 0));
-        for (int i : order_) f(i, lanes_[lane_of_[i]].s);
-        for (Lane& l : lanes_) {
-            MF3D_CK(cudaEventRecord(l.done, l.s));
-            MF3D_CK(cudaStreamWaitEvent(s_, l.done, 0));
-        }
+        then_always(
+            [&] {
+                for (Lane& l : lanes_) MF3D_CK(cudaStreamWaitEvent(l.s, fork_, 0));
+                for (int i : order_) f(i, lanes_[lane_of_[i]].s);
+            },
+            [&](bool failed) {
+                each_then_throw(lanes_.size(), [&](size_t k) {
+                    MF3D_CK(cudaEventRecord(lanes_[k].done, lanes_[k].s));
+                    MF3D_CK(cudaStreamWaitEvent(s_, lanes_[k].done, 0));
+                });
+                if (failed) MF3D_CK(cudaStreamSynchronize(s_));
+            });
     }
     void release() {
         for (Lane& l : lanes_) {

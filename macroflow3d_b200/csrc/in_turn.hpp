@@ -18,4 +18,20 @@ template <class F> void each_then_throw(size_t n, F&& f) {
     if (first) std::rethrow_exception(first);
 }
 
+// f(), then after(failed) whether f threw or not; f's exception is thrown rather than one of after's
+template <class F, class A> void then_always(F&& f, A&& after) {
+    std::exception_ptr first;
+    try {
+        f();
+    } catch (...) {
+        first = std::current_exception();
+    }
+    try {
+        after(first != nullptr);
+    } catch (...) {
+        if (!first) throw;
+    }
+    if (first) std::rethrow_exception(first);
+}
+
 } // namespace mf3d
