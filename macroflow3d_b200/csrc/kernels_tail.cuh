@@ -197,14 +197,15 @@ __device__ __forceinline__ void tail2_body(const Tail2Args& a, const TI* __restr
         a, [&](int c) { return (double)b_in[c]; }, [&](int c, double v) { x_out[c] = (TO)v; }, false);
 }
 
-// ---- the levels of at most kDenseMax cells as one matrix ----
+// ---- the coarsest levels as one matrix (VCycle::dense_level chooses the first of them) ----
 // From x = 0 the V-cycle on a level is a linear map of its b: dense_map_kernel runs the tail's own cycle
 // on every unit vector when K is set (one CTA per cell, its x is the column) and dense_apply_kernel applies
 // the matrix, a row per warp, instead of some hundred dependent half-sweeps.  The result is the cycle's up
 // to rounding, in FP64.  512 cells (2 MB): 2.8 us from L2, 5.5 from memory, the map 57 us a K; 960 cells 10 us; the
 // cluster kernel takes 25 us from 16^3 and 57 us from 24 x 20 x 16 cells, the one-CTA tail 150 us.
-constexpr int DN_MAX = 1024;      // cells of the first level that is solved this way
-constexpr int DN_MAX_LAST = 2048; // ... when it is the coarsest one, whose sweeps are many
+// cells of the first level that is solved this way, at most: with levels below it, when it is the coarsest one
+// (of at least DN_SWEEPS sweeps), and where what would serve otherwise is slow
+constexpr int DN_MAX = 512, DN_MAX_LAST = 384, DN_SWEEPS = 20, DN_MAX_SLOW = 1024;
 constexpr int DN_NT = 128; // threads per unit vector: cheap barriers, and every vector of 8^3 cells resident at once
 __global__ void __launch_bounds__(DN_NT, 8) dense_map_kernel(const Tail2Args a, int ld, double* __restrict__ M) {
     const int col = blockIdx.x;

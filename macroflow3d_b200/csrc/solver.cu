@@ -1075,17 +1075,29 @@ template <class T, class TC> class VCycle : public VCycleBase {
     bool cluster_on() const { return cp_.Lc >= 0 && !rec_tail_ && !rec_; }
     int coarse_start() const { return cluster_on() ? cp_.Lc : Lt_; }
     // ---- the FP64 levels of a single solve as bricks and one matrix ----
-    // The levels from the first FP64 one down to D_ (the first of at most DN_MAX cells, or the coarsest one of
-    // at most DN_MAX_LAST) run their legs in bricks, and the cycle from D_ on is a matrix product.  Where
-    // neither size fits, or other sweep counts need a level of legs, the cluster kernel or the one-CTA tail
-    // serves.
+    // The levels from the first FP64 one down to D_ run their legs in bricks, and the cycle from D_ on is a
+    // matrix product.  Where no level qualifies, or other sweep counts need a level of legs, the cluster kernel
+    // or the one-CTA tail serves.
+    //
+    // The matrix costs a cycle per cell when K is set and saves time in every V-cycle, so it has to pay within
+    // the solve's own cycles: 8 or 9 to 1e-10, 5 or 6 to 1e-6 (set_K, solve in ms; with the matrix | the cluster).
+    // D_ with levels below it, 50 coarsest sweeps: 512 cells (64^3) 0.15 + 0.92 | 0.13 + 1.00.  D_ the coarsest level:
+    // 216 cells 0.10 + 0.50 | 0.05 + 0.63, 343 cells 0.14 + 0.46 | 0.05 + 0.61, 512 cells 0.17 + 0.50 | 0.05 + 0.65 (paid
+    // after 4, 5 and 7 cycles), 1000 cells 0.44 + 0.68 | 0.05 + 0.94 (14 cycles), 1728 cells 1.11 + 0.42 | 0.04 + 0.90 (20
+    // cycles); 216 cells with 5 sweeps 0.06 + 0.59 | 0.05 + 0.58.  A grid that is one level needs 1 to 3 cycles when
+    // its sweeps are many: 343 cells, 400 sweeps 0.68 + 0.08 | 0.02 + 0.24.  The one-CTA tail, and the cluster where a
+    // coarsest level has more cells of a colour than threads, take 100 us a cycle instead of 30 to 60: a larger
+    // matrix pays there (9 x 11 x 10 cells 0.55 + 0.76 | 0.05 + 1.56).
     int dense_level(int nl) const { // D_, or -1
-        const int Ls = cp_.Lc >= 0 ? cp_.Lc : Lt_;
-        if (std::getenv("MF3D_NO_CLUSTER_TAIL")) return -1;
+        const bool cluster = cp_.Lc >= 0;
+        const int Ls = cluster ? cp_.Lc : Lt_;
+        if (nl == 1 || std::getenv("MF3D_NO_CLUSTER_TAIL") || std::getenv("MF3D_NO_MATRIX")) return -1;
+        const bool kept = cluster && cp_.a.L[cp_.a.nlev - 1].hcap <= CT_NT; // its sweeps run from registers
         int D = Ls;
-        while (D < nl && G_[D].n > (size_t)DN_MAX) ++D;
-        if (D == nl && G_[nl - 1].n <= (size_t)DN_MAX_LAST) D = nl - 1;
-        if (D == nl || D < Lt_ || (D > Ls && !(pre_ == 2 && post_ == 2))) return -1;
+        while (D < nl - 1 && G_[D].n > (size_t)(cluster ? DN_MAX : DN_MAX_SLOW)) ++D;
+        if (D == nl - 1 && (G_[D].n > (size_t)(kept ? DN_MAX_LAST : DN_MAX_SLOW) || (cluster && coarse_ < DN_SWEEPS)))
+            return -1;
+        if (D < Lt_ || (D > Ls && !(pre_ == 2 && post_ == 2))) return -1;
         size_t smem = 0; // of the cycle that builds the matrix
         for (int l = D; l < nl; ++l) smem += 8 * ((size_t)(G_[l].nx + 2) * (G_[l].ny + 2) * (G_[l].nz + 2) + G_[l].n);
         return smem > kDenseSmemMax ? -1 : D;

@@ -680,3 +680,44 @@ def test_coarse_end_ways_match_one_cta_tail(mf3d, monkeypatch, shape, levels, pe
         s.close()
     monkeypatch.delenv("MF3D_NO_CLUSTER_TAIL", raising=False)
     assert _rel(z[0], z[1]) < (1e-12 if prec == "fp64" else 1e-5)
+
+
+def _coarse_way(s):
+    """The way that the FP64 levels of a single solve go: the name of its entry in the profile."""
+    return [name for name, *_ in s.profile(1) if name.startswith("coarse_")]
+
+
+# where the matrix of the coarsest levels pays within a solve's own cycles and where it does not: too many cells
+# (1728; 512 whose cluster sweeps run from registers), a grid that is one level, few sweeps; at the limits (343 cells;
+# 512 with levels below; 990 with more cells of a colour than the cluster has threads, and 990 with fewer)
+@pytest.mark.parametrize("shape,levels,sweeps,way", [
+    ((24, 24, 24), 2, 50, "cluster"), ((8, 16, 16), 1, 400, "cluster"), ((7, 7, 7), 1, 50, "cluster"),
+    ((32, 32, 32), 3, 50, "cluster"), ((28, 28, 28), 3, 5, "cluster"), ((36, 44, 40), 3, 50, "cluster"),
+    ((28, 28, 28), 3, 50, "bricks_matrix"), ((28, 28, 28), 3, 20, "bricks_matrix"),
+    ((64, 64, 64), 16, 50, "bricks_matrix"), ((20, 20, 20), 3, 50, "bricks_matrix"),
+    ((40, 44, 36), 3, 50, "bricks_matrix")])
+def test_matrix_where_it_pays(mf3d, monkeypatch, shape, levels, sweeps, way):
+    """The way chosen, its memory (a matrix of at most 1024 x 1024), and the V-cycle against the cluster's: the same
+    cycle summed in another order, equal to rounding (1e-12 of the largest value)."""
+    M = mf3d
+    rng = np.random.default_rng(sum(shape) + levels + sweeps)
+    K, r = np.exp(rng.normal(size=shape)), rng.normal(size=shape)
+    g = M.Grid3D(shape[2], shape[1], shape[0], 0.5)
+    cfg = M.HeadSolveConfig(mg_levels=levels, mg_coarse_iters=sweeps)
+    z, size = [], []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("MF3D_NO_MATRIX", "1")
+        s = M.HeadSolver(g, M.BCSpec.darcy_x(), cfg)
+        s.set_K(_t(K))
+        zz = _t(np.zeros(shape))
+        s.vcycle(_t(r), zz)
+        z.append(_np(zz))
+        size.append(s.device_bytes)
+        assert _coarse_way(s) == ["coarse_" + ("cluster" if off else way)]
+        s.close()
+    monkeypatch.delenv("MF3D_NO_MATRIX", raising=False)
+    assert _rel(z[0], z[1]) < 1e-12
+    assert size[0] - size[1] <= (10 << 20)
+    if way == "cluster":
+        assert size[0] == size[1]
