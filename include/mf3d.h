@@ -323,9 +323,15 @@ int mf3d_init_head_guess(const mf3d_grid* g, const mf3d_bc* bc, double* h, void*
  * k1[n], k2[n], k3[n], a[n], b[n]; counter-based (Philox4x32-10) stream from `seed`. */
 int mf3d_kfield_modes(unsigned long long seed, int n_modes, int covariance, double lambda_x,
                       double lambda_y, double lambda_z, double* modes_host);
-/* K (or lnK when want_exp = 0) at the cell centres of g from device-resident modes. */
+/* K (or lnK when want_exp = 0) at the cell centres of g from device-resident modes.  Takes up to 32 MiB of
+ * device memory for the call, less or none where the device has none left. */
 int mf3d_kfield_eval(const mf3d_grid* g, int n_modes, const double* modes_dev, double sigma2,
                      double log_kg, int want_exp, double* out_dev, void* stream);
+/* Diagnostics: the same field in parts of at most axis_cells cells along each axis, with at most table_bytes of
+ * device memory (or 8 modes' tables; 0: none), as very long axes, very many modes or a full device have it. */
+int mf3d_diag_kfield_parts(const mf3d_grid* g, int n_modes, const double* modes_dev, double sigma2,
+                           double log_kg, int want_exp, long long table_bytes, int axis_cells, double* out_dev,
+                           void* stream);
 
 #ifdef __cplusplus
 }

@@ -105,6 +105,8 @@ SIGNATURES = {
     "mf3d_init_head_guess": ([_G, _B, _P, _P], C.c_int),
     "mf3d_kfield_modes": ([C.c_ulonglong, C.c_int, C.c_int, C.c_double, C.c_double, C.c_double,
                            C.POINTER(C.c_double)], C.c_int),
+    "mf3d_diag_kfield_parts": ([_G, C.c_int, _P, C.c_double, C.c_double, C.c_int, C.c_longlong, C.c_int, _P, _P],
+                               C.c_int),
     "mf3d_kfield_eval": ([_G, C.c_int, _P, C.c_double, C.c_double, C.c_int, _P, _P], C.c_int),
 }
 

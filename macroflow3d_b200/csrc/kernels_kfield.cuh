@@ -171,4 +171,26 @@ __global__ void __launch_bounds__(KF_NT) kfield_kernel(const KfPart w, int mp, i
     }
 }
 
+// The same part without tables, a cell per thread: where the device has no room for them (a sine and a cosine per
+// mode and cell).
+__global__ void __launch_bounds__(256) kfield_direct_kernel(const KfPart w, double dx, int n_modes,
+                                                            const double* __restrict__ modes, double scale,
+                                                            double log_kg, int want_exp, double* __restrict__ out) {
+    const size_t n = (size_t)w.nx * w.ny * w.nz;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+        const int i = w.ox + (int)(e % w.nx), j = w.oy + (int)((e / w.nx) % w.ny), k = w.oz + (int)(e / ((size_t)w.nx * w.ny));
+        const double x = dx * (i + 0.5), y = dx * (j + 0.5), z = dx * (k + 0.5);
+        double v = 0.0;
+        for (int m = 0; m < n_modes; ++m) {
+            const double* q = modes + m;
+            double s, c;
+            sincos(q[0] * x + q[(size_t)n_modes] * y + q[2 * (size_t)n_modes] * z, &s, &c);
+            v += q[3 * (size_t)n_modes] * s + q[4 * (size_t)n_modes] * c;
+        }
+        v *= scale;
+        if (want_exp) v = exp(v + log_kg);
+        out[(size_t)i + (size_t)w.NX * ((size_t)j + (size_t)w.NY * k)] = v;
+    }
+}
+
 } // namespace mf3d

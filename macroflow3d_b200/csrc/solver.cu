@@ -114,6 +114,8 @@ static ColLaunch col_launch_staged(int nx, int ny, int nz, int per_sm) {
     return col_launch(nx, ny, nz, per_sm);
 }
 
+static bool trim_scratch_pool();
+
 // RAII device allocation
 struct DevMem {
     void* p = nullptr;
@@ -123,7 +125,13 @@ struct DevMem {
     void alloc(size_t b) {
         release();
         bytes = b;
-        if (b) MF3D_CK(cudaMalloc(&p, b));
+        if (!b) return;
+        cudaError_t e = cudaMalloc(&p, b);
+        if (e == cudaErrorMemoryAllocation && trim_scratch_pool()) {
+            cudaGetLastError(); // (the failure that has been handled)
+            e = cudaMalloc(&p, b);
+        }
+        MF3D_CK(e);
     }
     void release() {
         if (p) cudaFree(p);
@@ -137,29 +145,40 @@ struct DevMem {
 };
 
 // Scratch of one call, in stream order, from a pool of this library: cudaMalloc and cudaFree cost a call
-// 0.6 ms (they synchronise the device).  The pool keeps at most kScratchKeep bytes between calls and is
-// the driver's own, so calls on several threads and streams may use it at once.
-static constexpr unsigned long long kScratchKeep = 64ull << 20;
-static cudaMemPool_t scratch_pool() {
+// 0.6 ms (they synchronise the device).  The pool keeps at most kScratchKeep bytes between calls, gives them back
+// when an allocation of this library finds the device full, and is the driver's own, so calls on several threads
+// and streams may use it at once.
+static constexpr unsigned long long kScratchKeep = 32ull << 20;
+static std::mutex g_pool_mu;
+static cudaMemPool_t* scratch_pool_slot() { // of the current device (under g_pool_mu)
     constexpr int kDevices = 64;
-    static std::mutex mu;
     static cudaMemPool_t pools[kDevices] = {};
     int dev = 0;
     MF3D_CK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kDevices) throw Error(MF3D_E_INVALID, "device ordinal out of range for the scratch pool");
-    std::lock_guard<std::mutex> lock(mu);
-    if (!pools[dev]) {
+    return &pools[dev];
+}
+static cudaMemPool_t scratch_pool() {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    cudaMemPool_t* pool = scratch_pool_slot();
+    if (!*pool) {
         cudaMemPoolProps pr{};
         pr.allocType = cudaMemAllocationTypePinned;
         pr.location.type = cudaMemLocationTypeDevice;
-        pr.location.id = dev;
+        MF3D_CK(cudaGetDevice(&pr.location.id));
         cudaMemPool_t p;
         MF3D_CK(cudaMemPoolCreate(&p, &pr));
         unsigned long long keep = kScratchKeep;
         MF3D_CK(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
-        pools[dev] = p;
+        *pool = p;
     }
-    return pools[dev];
+    return *pool;
+}
+// gives the pool's unused memory back to the device; false when there is no pool
+static bool trim_scratch_pool() {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    cudaMemPool_t* pool = scratch_pool_slot();
+    return *pool && cudaMemPoolTrimTo(*pool, 0) == cudaSuccess;
 }
 struct StreamMem {
     void* p = nullptr;
@@ -2623,6 +2642,14 @@ int mf3d_kfield_modes(unsigned long long seed, int n_modes, int cov, double lx, 
     });
 }
 
+// A part without tables
+static void kfield_direct(KfPart w, double dx, int n_modes, const double* modes, double scale, double log_kg,
+                          int want_exp, double* out, cudaStream_t s) {
+    const size_t n = (size_t)w.nx * w.ny * w.nz;
+    kfield_direct_kernel<<<grid1d(n, 256), 256, 0, s>>>(w, dx, n_modes, modes, scale, log_kg, want_exp, out);
+    MF3D_LAUNCH_CK();
+}
+
 // The modes of one part, in batches whose tables take at most `table` bytes (or 8 modes).
 static void kfield_part(KfPart w, double dx, int n_modes, const double* modes, double scale, double log_kg,
                         int want_exp, double* out, size_t table, cudaStream_t s) {
@@ -2656,31 +2683,60 @@ static void kfield_part(KfPart w, double dx, int n_modes, const double* modes, d
     }
 }
 
+// The field in parts of at most `axis` cells along each axis, with tables of at most `table` bytes (or 8 modes;
+// 0: none).  Where the device has no room for the tables they get smaller, down to none at all: a field needs no
+// memory but its own.
+static void kfield_eval(const mf3d_grid* g, int n_modes, const double* modes, double sigma2, double log_kg,
+                        int want_exp, double* out, size_t table, int axis, cudaStream_t s) {
+    check_grid(g);
+    need(modes, "modes");
+    need(out, "out");
+    if (n_modes <= 0 || sigma2 < 0) throw Error(MF3D_E_INVALID, "bad n_modes or variance");
+    const double scale = std::sqrt(sigma2) / std::sqrt((double)n_modes);
+    auto part = [&](const KfPart& w) {
+        size_t room = table;
+        while (room > 0) {
+            try {
+                kfield_part(w, g->dx, n_modes, modes, scale, log_kg, want_exp, out, room, s);
+                return;
+            } catch (const Error& e) { // (the tables are made before anything is launched)
+                if (e.code != MF3D_E_NOMEM) throw;
+                cudaGetLastError();
+                trim_scratch_pool();
+                const size_t least = (size_t)KF_MC * 2 * sizeof(double) * ((size_t)w.nx + 64 + w.ny + w.nz);
+                room = room > least ? std::max(room / 8, least) : 0;
+            }
+        }
+        kfield_direct(w, g->dx, n_modes, modes, scale, log_kg, want_exp, out, s);
+    };
+    KfPart w{};
+    w.NX = g->nx;
+    w.NY = g->ny;
+    for (w.oz = 0; w.oz < g->nz; w.oz += axis)
+        for (w.oy = 0; w.oy < g->ny; w.oy += axis)
+            for (w.ox = 0; w.ox < g->nx; w.ox += axis) {
+                w.nx = std::min(axis, g->nx - w.ox);
+                w.ny = std::min(axis, g->ny - w.oy);
+                w.nz = std::min(axis, g->nz - w.oz);
+                part(w);
+            }
+    MF3D_CK(cudaStreamSynchronize(s));
+}
+
 int mf3d_kfield_eval(const mf3d_grid* g, int n_modes, const double* modes, double sigma2, double log_kg,
                      int want_exp, double* out, void* stream) {
+    // one part in ordinary use (1000 modes of 600^3 cells are 29 MB of tables); a very long axis or very many
+    // modes go in several, each a pass over the field more
     return guard([&] {
-        check_grid(g);
-        need(modes, "modes");
-        need(out, "out");
-        if (n_modes <= 0 || sigma2 < 0) throw Error(MF3D_E_INVALID, "bad n_modes or variance");
-        cudaStream_t s = (cudaStream_t)stream;
-        const double scale = std::sqrt(sigma2) / std::sqrt((double)n_modes);
-        // one part in ordinary use; a very long axis or very many modes go in several, so that the tables stay
-        // below 256 MiB (or 8 modes)
-        constexpr int kAxis = 1 << 20;
-        constexpr size_t kTable = 256ull << 20;
-        KfPart w{};
-        w.NX = g->nx;
-        w.NY = g->ny;
-        for (w.oz = 0; w.oz < g->nz; w.oz += kAxis)
-            for (w.oy = 0; w.oy < g->ny; w.oy += kAxis)
-                for (w.ox = 0; w.ox < g->nx; w.ox += kAxis) {
-                    w.nx = std::min(kAxis, g->nx - w.ox);
-                    w.ny = std::min(kAxis, g->ny - w.oy);
-                    w.nz = std::min(kAxis, g->nz - w.oz);
-                    kfield_part(w, g->dx, n_modes, modes, scale, log_kg, want_exp, out, kTable, s);
-                }
-        MF3D_CK(cudaStreamSynchronize(s));
+        kfield_eval(g, n_modes, modes, sigma2, log_kg, want_exp, out, (size_t)kScratchKeep, 1 << 16, (cudaStream_t)stream);
+    });
+}
+
+int mf3d_diag_kfield_parts(const mf3d_grid* g, int n_modes, const double* modes, double sigma2, double log_kg,
+                           int want_exp, long long table_bytes, int axis_cells, double* out, void* stream) {
+    return guard([&] {
+        if (table_bytes < 0 || axis_cells < 1) throw Error(MF3D_E_INVALID, "bad table size or part length");
+        kfield_eval(g, n_modes, modes, sigma2, log_kg, want_exp, out, (size_t)table_bytes, axis_cells, (cudaStream_t)stream);
     });
 }
 

@@ -721,3 +721,50 @@ def test_matrix_where_it_pays(mf3d, monkeypatch, shape, levels, sweeps, way):
     assert size[0] - size[1] <= (10 << 20)
     if way == "cluster":
         assert size[0] == size[1]
+
+
+# several batches of modes (the last one ragged), several parts along one axis or all (ragged, of one cell), no
+# tables at all
+@pytest.mark.parametrize("shape,modes,table,axis", [((9, 14, 70), 50, 1, 1 << 16), ((21, 17, 33), 100, 3 * 8 * 16 * 102, 1 << 16),
+                                                    ((20, 7, 150), 37, 1 << 20, 64), ((23, 40, 9), 24, 1 << 20, 11),
+                                                    ((33, 20, 70), 41, 1, 32), ((5, 3, 4), 9, 1, 1),
+                                                    ((9, 14, 70), 50, 0, 1 << 16), ((23, 40, 9), 24, 0, 11)])
+def test_kfield_in_parts_vs_numpy(mf3d, shape, modes, table, axis):
+    """lnK and K from every split of a field against the sum over the modes (as in the test of the tile shapes)."""
+    import ctypes as C
+    import torch
+    M = mf3d
+    from macroflow3d_b200 import _lib
+    g = M.Grid3D(shape[2], shape[1], shape[0], 0.7)
+    tab = M.kfield_modes(5, modes, M.COV_EXPONENTIAL, (4.0, 3.0, 2.0))
+    x = [(np.arange(n) + 0.5) * 0.7 for n in (shape[2], shape[1], shape[0])]
+    ref = np.zeros(shape)
+    for k1, k2, k3, a, b in tab.T:
+        ph = (k3 * x[2])[:, None, None] + (k2 * x[1])[None, :, None] + (k1 * x[0])[None, None, :]
+        ref += a * np.sin(ph) + b * np.cos(ph)
+    ref *= np.sqrt(1.5 / modes)
+    dev = torch.from_numpy(np.ascontiguousarray(tab)).cuda()
+    for want_exp in (0, 1):
+        out = torch.full(shape, float("nan"), dtype=torch.float64, device="cuda")
+        M.check(_lib.lib().mf3d_diag_kfield_parts(C.byref(g.c()), modes, dev.data_ptr(), 1.5, float(np.log(2.0)), want_exp,
+                                                  table, axis, out.data_ptr(), 0))
+        if want_exp:
+            assert np.allclose(_np(out), 2.0 * np.exp(ref), rtol=1e-9)
+        else:
+            assert np.abs(_np(out) - ref).max() < 1e-10
+
+
+def test_kfield_keeps_little_device_memory(mf3d):
+    """Tables of a 65536-cell axis and 2000 modes (2.1 GB at once) go in batches: the library keeps no more than
+    32 MiB of the device afterwards, and 40 MiB with what the driver rounds up."""
+    import torch
+    M = mf3d
+    g = M.Grid3D(65536, 4, 2, 0.7)
+    M.generate_K_field(M.Grid3D(64, 4, 2, 0.7), 1.0, seed=1, n_modes=8)  # (context, module and pool)
+    torch.cuda.synchronize()
+    out = torch.empty((2, 4, 65536), dtype=torch.float64, device="cuda")
+    del out  # (the cached block that the call below takes)
+    free = torch.cuda.mem_get_info()[0]
+    lnk = M.generate_K_field(g, 1.0, (4.0, 4.0, 4.0), seed=3, n_modes=2000, log_only=True)
+    assert bool(torch.isfinite(lnk).all())
+    assert free - torch.cuda.mem_get_info()[0] <= 40 << 20
