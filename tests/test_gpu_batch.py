@@ -1,6 +1,6 @@
 """Batched ensemble solves (mf3d_batch_*) against one HeadSolver per realisation.
 
-The batch replaces the realisation loop of run_ensemble (src/runtime/ensemble/
+A batch replaces the realisation loop of run_ensemble (src/runtime/ensemble/
 EnsembleRunner.cu:259-317), so every realisation must come out as its own single solve would:
 same iteration count (the batch changes only the summation order of the in-sweep <r, z>), the
 same head to well below the solve tolerance, and the per-realisation stopping test must freeze
@@ -59,6 +59,12 @@ def _single(M, grids, bc, cfg, Ks):
         out.append((h.cpu().numpy(), res))
         s.close()
     return out
+
+
+def _assert_batched(b):
+    """The realisations are solved by batched launches: only these have sweeps to tune (ensembles of at most four
+    small realisations, and large ones, are solved side by side by their own launches)."""
+    assert b.autotune(1), "no realisation is batched"
 
 
 def _batch(M, grids, bc, cfg, Ks, tune=False, x0s=None):
@@ -120,20 +126,27 @@ def test_convergence_mask_freezes_finished_realisations(mf3d):
     easy realisation must report its own count and keep its own converged head."""
     import torch
     M = mf3d
-    grids = [M.Grid3D(32, 32, 32, 1.0), M.Grid3D(48, 32, 32, 1.0), M.Grid3D(32, 48, 64, 1.0)]
+    grids = [M.Grid3D(32, 32, 32, 1.0), M.Grid3D(48, 32, 32, 1.0), M.Grid3D(32, 48, 64, 1.0),
+             M.Grid3D(32, 32, 40, 1.0), M.Grid3D(40, 32, 32, 1.0)]
     bc = M.BCSpec.darcy_x()
     cfg = _cfg(M, M.PREC_FP32)
     Ks = [torch.ones((32, 32, 32), dtype=torch.float64, device="cuda"),
           M.generate_K_field(grids[1], 4.0, (8.0, 8.0, 8.0), seed=5),
-          M.generate_K_field(grids[2], 1.0, (4.0, 4.0, 4.0), seed=6)]
-    ref = _single(M, grids, bc, cfg, Ks)
-    its = [r.num_iterations for _, r in ref]
-    assert its[0] < its[1] - 3, its
-    b, got, _ = _batch(M, grids, bc, cfg, Ks)
-    for (hr, rr), (hb, rb) in zip(ref, got):
-        assert rb.converged and abs(rb.num_iterations - rr.num_iterations) <= 1
-        assert _rel(hb, hr) < HEAD_TOL
-    b.close()
+          M.generate_K_field(grids[2], 1.0, (4.0, 4.0, 4.0), seed=6),
+          torch.ones((40, 32, 32), dtype=torch.float64, device="cuda"),
+          M.generate_K_field(grids[4], 4.0, (8.0, 8.0, 8.0), seed=7)]
+    for few in (False, True):  # all five as one batch; three of them side by side
+        n = 3 if few else 5
+        ref = _single(M, grids[:n], bc, cfg, Ks[:n])
+        its = [r.num_iterations for _, r in ref]
+        assert its[0] < its[1] - 3, its
+        b, got, _ = _batch(M, grids[:n], bc, cfg, Ks[:n])
+        for (hr, rr), (hb, rb) in zip(ref, got):
+            assert rb.converged and abs(rb.num_iterations - rr.num_iterations) <= 1
+            assert _rel(hb, hr) < HEAD_TOL
+        if not few:
+            _assert_batched(b)
+        b.close()
 
 
 def test_autotune_keeps_results(mf3d):
@@ -161,9 +174,11 @@ def test_autotune_keeps_results(mf3d):
     b1.close()
 
 
-def test_host_loop_equals_graph(mf3d):
+@pytest.mark.parametrize("count", [5, 3])
+def test_host_loop_equals_graph(mf3d, count):
+    """Five realisations are one batch (its loop driven by the host polls the gate), three are side by side."""
     M = mf3d
-    grids = _grids(M)[:3]
+    grids = _grids(M)[:count]
     bc = M.BCSpec.darcy_x()
     Ks = _fields(M, grids, seed=400)
     bg, g, _ = _batch(M, grids, bc, _cfg(M, M.PREC_FP32), Ks)
@@ -171,24 +186,30 @@ def test_host_loop_equals_graph(mf3d):
     for (ha, ra), (hb, rb) in zip(g, h):
         assert ra.num_iterations == rb.num_iterations
         assert np.array_equal(ha, hb)
+    if count == 5:
+        _assert_batched(bg)
+        _assert_batched(bh)
     bg.close()
     bh.close()
 
 
-def test_warm_start_and_iteration_cap(mf3d):
+@pytest.mark.parametrize("count", [5, 3])
+def test_warm_start_and_iteration_cap(mf3d, count):
     """x0 per realisation (None entries use the reference guess); a cap of 3 iterations stops
-    every realisation unconverged with 3 iterations."""
+    every realisation unconverged with 3 iterations.  Five realisations are one batch, three are side by side."""
     import torch
     M = mf3d
-    grids = _grids(M)[:3]
+    grids = _grids(M)[:count]
     bc = M.BCSpec.darcy_x()
     Ks = _fields(M, grids, seed=500)
     b, got, _ = _batch(M, grids, bc, _cfg(M, M.PREC_FP32), Ks)
-    x0s = [torch.from_numpy(got[0][0]).cuda(), None, torch.from_numpy(got[2][0]).cuda()]
+    x0s = [torch.from_numpy(got[0][0]).cuda(), None, torch.from_numpy(got[2][0]).cuda()] + [None] * (count - 3)
     hs = [torch.empty_like(K) for K in Ks]
     res = b.solve(hs, x0s)
     assert res[0].num_iterations <= 1 and res[2].num_iterations <= 1
-    assert res[1].num_iterations == got[1][1].num_iterations
+    assert all(res[r].num_iterations == got[r][1].num_iterations for r in range(count) if x0s[r] is None)
+    if count == 5:
+        _assert_batched(b)
     b.close()
     bcap, capped, _ = _batch(M, grids, bc, _cfg(M, M.PREC_FP32, cg_max_iter=3), Ks)
     for _, r in capped:
@@ -196,21 +217,26 @@ def test_warm_start_and_iteration_cap(mf3d):
     bcap.close()
 
 
-def test_nonfinite_realisation_does_not_stop_the_others(mf3d):
+@pytest.mark.parametrize("count", [5, 3])
+def test_nonfinite_realisation_does_not_stop_the_others(mf3d, count):
+    """Five realisations are one batch, three are side by side."""
     import torch
     M = mf3d
-    grids = _grids(M)[:3]
+    grids = _grids(M)[:count]
     bc = M.BCSpec.darcy_x()
     cfg = _cfg(M, M.PREC_FP32)
     Ks = _fields(M, grids, seed=600)
     Ks[1] = Ks[1].clone()
     Ks[1].view(-1)[17] = float("nan")
-    ref = _single(M, [grids[0], grids[2]], bc, cfg, [Ks[0], Ks[2]])
+    rest = [r for r in range(count) if r != 1]
+    ref = _single(M, [grids[r] for r in rest], bc, cfg, [Ks[r] for r in rest])
     b, got, _ = _batch(M, grids, bc, cfg, Ks)
     assert got[1][1].status == 2 and not got[1][1].converged
-    for (hr, rr), (hb, rb) in zip(ref, [got[0], got[2]]):
+    for (hr, rr), (hb, rb) in zip(ref, [got[r] for r in rest]):
         assert rb.converged and abs(rb.num_iterations - rr.num_iterations) <= 1
         assert _rel(hb, hr) < HEAD_TOL
+    if count == 5:
+        _assert_batched(b)
     b.close()
 
 
@@ -226,7 +252,7 @@ def test_guesses_in_other_realisations_heads(mf3d):
     cfg = _cfg(M, M.PREC_FP64)
     Ks = _fields(M, grids, seed=900)
     b, got, _ = _batch(M, grids, bc, cfg, Ks)
-    assert b.autotune(1), "no realisation is batched"
+    _assert_batched(b)
     heads = [torch.from_numpy(h).cuda() for h, _ in got]
     hs = [torch.empty_like(K) for K in Ks]
     x0s = [None] * len(grids)
@@ -321,7 +347,7 @@ def test_reductions_of_successive_blocks_do_not_mix(mf3d):
     Kb = _fields(M, base, seed=800)
     grids, Ks = base * 32, Kb * 32
     b, first, _ = _batch(M, grids, M.BCSpec.darcy_x(), _cfg(M, M.PREC_FP64, cg_max_iter=30), Ks)
-    assert b.autotune(1), "the realisations are not batched"
+    _assert_batched(b)
     hs = [torch.empty_like(K) for K in Ks]
     b.solve(hs)  # (with the tuned sweeps, repeated below)
     tuned = None
@@ -386,19 +412,25 @@ def test_mixed_sizes_keep_their_places(mf3d, prec):
     b.close()
 
 
+@pytest.mark.parametrize("way", ["batched", "side_by_side"])
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
-def test_batch_vs_oracle(mf3d, oracle_mod, prec):
-    """Three uneven realisations (non-cubic coarse grids) solved as one batch, each against the
-    FP64 oracle at the same tolerance (the realisation loop the batch replaces:
+def test_batch_vs_oracle(mf3d, oracle_mod, prec, way):
+    """Uneven realisations (non-cubic coarse grids), five small ones solved as one batch or three large ones side
+    by side, each against the FP64 oracle at the same tolerance (the realisation loop the batch replaces:
     src/runtime/ensemble/EnsembleRunner.cu:259-317).  FP64: the reference algorithm, same
     iteration count, heads equal to rounding (measured 1e-14).  FP32 V-cycle: iterations within
     one, heads within the tolerance's reach (measured 1.2e-9)."""
     M, O = mf3d, oracle_mod
-    shapes = [(64, 96, 64), (96, 64, 128), (128, 64, 96)]
+    shapes = {"batched": [(32, 48, 64), (48, 32, 64), (64, 32, 48), (64, 48, 32), (32, 32, 32)],
+              "side_by_side": [(64, 96, 64), (96, 64, 128), (128, 64, 96)]}[way]
     grids = [M.Grid3D(*s) for s in shapes]
     Ks = _fields(M, grids, seed=500)
     cfg = _cfg(M, getattr(M, "PREC_" + prec.upper()))
     b, out, _ = _batch(M, grids, M.BCSpec.darcy_x(), cfg, Ks)
+    if way == "batched":
+        _assert_batched(b)
+    else:
+        assert not b.autotune(1)
     b.close()
     bc = O.baseline_bc()
     for (h, res), K, g in zip(out, Ks, grids):
