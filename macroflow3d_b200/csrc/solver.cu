@@ -766,7 +766,8 @@ template <class T, class TC> class VCycle : public VCycleBase {
         }
         // levels whose legs run in bricks (kernels_brick.cuh): two sweeps a leg, and few enough bricks
         brick_.assign(Lt, 0);
-        for (int l = 0; l < Lt; ++l) {
+        const bool bricks = std::getenv("MF3D_NO_BRICKS") == nullptr; // (tests: sweeps on every level)
+        for (int l = 0; bricks && l < Lt; ++l) {
             const dim3 g = brick_grid(G[l]);
             brick_[l] = pre == 2 && post == 2 && (long long)g.x * g.y * g.z <= (long long)kBrickWaves * num_sms();
         }

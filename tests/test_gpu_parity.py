@@ -173,11 +173,13 @@ def test_vcycle_vs_oracle(mf3d, oracle_mod, shape, levels, pre, post, coarse, ca
                                           ((64, 48, 32), 4)])
 @pytest.mark.parametrize("bcname", ["darcy", "periodic_yz"])
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
-def test_cluster_coarse_end_matches_one_cta_tail(mf3d, monkeypatch, shape, levels, bcname, prec):
+@pytest.mark.parametrize("pre,post", [(2, 2), (1, 3)])
+def test_cluster_coarse_end_matches_one_cta_tail(mf3d, monkeypatch, shape, levels, bcname, prec, pre, post):
     """The coarse end in one thread-block cluster (levels of up to 32^3 cells in z slabs over
-    the cluster's CTAs, FP64) against the same V-cycle with the one-CTA tail and x-pair sweeps
-    above it: equal to rounding in FP64 (1e-12), to FP32 rounding of the levels it replaces
-    in the FP32 V-cycle (1e-5)."""
+    the cluster's CTAs, FP64; a coarsest level of at most 64 cells as its own map) against the same V-cycle
+    with the one-CTA tail and x-pair sweeps above it: equal to rounding in FP64 (1e-12), to FP32 rounding of
+    the levels it replaces in the FP32 V-cycle (1e-5).  The matrix of the coarsest levels, which would take the
+    cluster's place here, is off, and in the tail's arm the bricks."""
     M = mf3d
     rng = np.random.default_rng(zlib.crc32(repr((shape, levels, bcname)).encode()))
     K = np.exp(rng.normal(size=shape))
@@ -188,11 +190,11 @@ def test_cluster_coarse_end_matches_one_cta_tail(mf3d, monkeypatch, shape, level
     else:
         bc = _bcs(M, [D, D, P, P, P, P], [1.0, 0.0, 0, 0, 0, 0])
     P_ = {"fp64": M.PREC_FP64, "fp32": M.PREC_FP32}[prec]
-    cfg = M.HeadSolveConfig(mg_levels=levels, precision=P_)
+    cfg = M.HeadSolveConfig(mg_levels=levels, mg_pre_smooth=pre, mg_post_smooth=post, precision=P_)
     z = {}
-    for mode in ("cluster", "tail"):
-        if mode == "tail":
-            monkeypatch.setenv("MF3D_NO_CLUSTER_TAIL", "1")
+    for mode, off in (("cluster", ["MF3D_NO_MATRIX"]), ("tail", ["MF3D_NO_CLUSTER_TAIL", "MF3D_NO_BRICKS"])):
+        for name in off:
+            monkeypatch.setenv(name, "1")
         s = M.HeadSolver(g, bc, cfg)
         first, ctas = s.coarse_info
         if mode == "cluster":
@@ -203,8 +205,10 @@ def test_cluster_coarse_end_matches_one_cta_tail(mf3d, monkeypatch, shape, level
         zz = _t(np.zeros(shape))
         s.vcycle(_t(r), zz)
         z[mode] = _np(zz)
+        assert _coarse_way(s) == ["coarse_" + mode]
         s.close()
-        monkeypatch.delenv("MF3D_NO_CLUSTER_TAIL", raising=False)
+        for name in off:
+            monkeypatch.delenv(name)
     assert _rel(z["cluster"], z["tail"]) < (1e-12 if prec == "fp64" else 1e-5)
 
 
@@ -213,7 +217,9 @@ def test_cluster_coarse_end_matches_one_cta_tail(mf3d, monkeypatch, shape, level
 def test_bf16_vcycle_staged_matches_unstaged(mf3d, monkeypatch, shape, levels, bcname):
     """The BF16-coefficient V-cycle on the TMA-staged x-pair sweep and the staged residual +
     restriction against the same V-cycle on the unstaged sweep (MF3D_NO_TMA): the same BF16
-    coefficients and FP32 arithmetic, so equal to FP32 rounding (1e-5 of the max)."""
+    coefficients and FP32 arithmetic, so equal to FP32 rounding (1e-5 of the max).  Both arms sweep: small
+    levels would run in bricks, which stage nothing."""
+    monkeypatch.setenv("MF3D_NO_BRICKS", "1")
     M = mf3d
     rng = np.random.default_rng(zlib.crc32(repr((shape, levels, bcname, "bf16")).encode()))
     K = np.exp(rng.normal(size=shape))
@@ -231,6 +237,8 @@ def test_bf16_vcycle_staged_matches_unstaged(mf3d, monkeypatch, shape, levels, b
         zz = _t(np.zeros(shape))
         s.vcycle(_t(r), zz)
         z[mode] = _np(zz)
+        sweeps = {name.rsplit("_", 1)[1] for name, *_ in s.profile(1) if name.startswith("sweep_l0")}
+        assert sweeps == {"pair" if mode == "staged" else "ldg"}
         s.close()
         monkeypatch.delenv("MF3D_NO_TMA", raising=False)
     assert _rel(z["staged"], z["unstaged"]) < 1e-5
@@ -652,16 +660,17 @@ def test_velocity_and_diagnostics_edges_vs_numpy(mf3d, shape, per):
         assert np.allclose(s, (o.min(), o.max(), o.mean()), rtol=1e-11, atol=1e-11 * max(scale, scale ** 2))
 
 
-# the coarse end by its ways: bricks above a matrix with ragged bricks; the matrix alone from the coarsest level
-# of more than 1024 cells; the cluster with a cell of each colour per thread (6175 cells); an odd periodic
-# count on the coarsest level; a hierarchy that is one matrix
-@pytest.mark.parametrize("shape,levels,per", [((24, 40, 56), 4, False), ((20, 24, 28), 2, False),
-                                              ((26, 38, 50), 2, False), ((48, 96, 80), 5, True),
-                                              ((12, 20, 36), 3, True), ((8, 10, 12), 2, False)])
+# the coarse end by its ways: bricks above a matrix with ragged bricks; the cluster with a coarsest level of 1680
+# cells, and with a cell of each colour per thread (6175 cells); an odd periodic count on the coarsest level
+# (bricks and matrix); a matrix from the coarsest of two levels on; a hierarchy that is one matrix
+@pytest.mark.parametrize("shape,levels,per,way", [
+    ((24, 40, 56), 4, False, "bricks_matrix"), ((20, 24, 28), 2, False, "cluster"), ((26, 38, 50), 2, False, "cluster"),
+    ((48, 96, 80), 5, True, "bricks_matrix"), ((12, 20, 36), 3, True, "bricks_matrix"),
+    ((8, 10, 12), 2, False, "bricks_matrix"), ((8, 8, 8), 2, False, "bricks_matrix")])
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
-def test_coarse_end_ways_match_one_cta_tail(mf3d, monkeypatch, shape, levels, per, prec):
-    """Against the same V-cycle with sweeps down to the one-CTA tail: the same arithmetic in another order, so
-    equal to rounding (1e-12 in FP64, 1e-5 where FP32 levels are swept by another kernel)."""
+def test_coarse_end_ways_match_one_cta_tail(mf3d, monkeypatch, shape, levels, per, way, prec):
+    """Against the same V-cycle with sweeps down to the one-CTA tail (no bricks either): the same arithmetic in
+    another order, so equal to rounding (1e-12 in FP64, 1e-5 where FP32 levels are swept by another kernel)."""
     M = mf3d
     rng = np.random.default_rng(sum(shape) + levels)
     K, r = np.exp(rng.normal(size=shape)), rng.normal(size=shape)
@@ -672,13 +681,15 @@ def test_coarse_end_ways_match_one_cta_tail(mf3d, monkeypatch, shape, levels, pe
     for tail in (False, True):
         if tail:
             monkeypatch.setenv("MF3D_NO_CLUSTER_TAIL", "1")
+            monkeypatch.setenv("MF3D_NO_BRICKS", "1")
         s = M.HeadSolver(g, bc, cfg)
         s.set_K(_t(K))
         zz = _t(np.zeros(shape))
         s.vcycle(_t(r), zz)
         z.append(_np(zz))
+        assert _coarse_way(s) == ["coarse_" + ("tail" if tail else way)]
+        assert not tail or not [n for n, *_ in s.profile(1) if n.startswith("brick")]
         s.close()
-    monkeypatch.delenv("MF3D_NO_CLUSTER_TAIL", raising=False)
     assert _rel(z[0], z[1]) < (1e-12 if prec == "fp64" else 1e-5)
 
 
