@@ -545,11 +545,11 @@ __global__ void __launch_bounds__(PK_NT) mg_xupdate_kernel(size_t n, double* __r
         x[c] = x[c] + (double)z[c];
 }
 
-// Re-opens a finished state so the iteration kernels can be timed in isolation (diagnostics).
-__global__ void pcg_reopen_kernel(PcgState* st) {
+// Re-opens a finished state at an iteration so the iteration's kernels can be timed in isolation (diagnostics).
+__global__ void pcg_reopen_kernel(PcgState* st, int iter) {
     st->stop = 0;
     st->body_count = 0;
-    st->iter = 1;
+    st->iter = iter;
     st->rtol = 0.0; // never converges while being timed
     st->t_start_ns = global_ns();
 }

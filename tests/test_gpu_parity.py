@@ -779,3 +779,21 @@ def test_kfield_keeps_little_device_memory(mf3d):
     lnk = M.generate_K_field(g, 1.0, (4.0, 4.0, 4.0), seed=3, n_modes=2000, log_only=True)
     assert bool(torch.isfinite(lnk).all())
     assert free - torch.cuda.mem_get_info()[0] <= 40 << 20
+
+
+@pytest.mark.parametrize("prec,ez", [("fp64", 8), ("fp32", 4)])
+def test_profile_counts_the_head_update(mf3d, prec, ez):
+    """The profile's matvec is the mean over iterations with and without the two steps of the head update (24 bytes
+    a cell every second iteration, 12 on average), and a solve after it repeats the one before it."""
+    M = mf3d
+    n = (40, 48, 64)
+    s = M.HeadSolver(M.Grid3D(64, 48, 40, 1.0), M.BCSpec.darcy_x(),
+                     M.HeadSolveConfig(mg_levels=8, cg_rtol=1e-10, cg_check_every=1, precision=getattr(M, "PREC_" + prec.upper())))
+    s.set_K(_t(_lognormal(n, 1.0, 7)))
+    h0, h1 = _t(np.zeros(n)), _t(np.zeros(n))
+    r0 = s.solve(h0)
+    got = {name: (ms, nbytes, per) for name, ms, nbytes, per in s.profile(3)}["pupdate_matvec_dot"]
+    assert got[0] > 0 and got[1] == (60 + ez) * 64 * 48 * 40 and got[2] == 1
+    r1 = s.solve(h1)
+    assert r0.num_iterations == r1.num_iterations and np.array_equal(_np(h0), _np(h1))
+    s.close()
