@@ -247,3 +247,25 @@ def test_conv3d_ring_and_channel_splits_vs_oracle(mf3d, shape, cin, cout):
     y = M.nn_conv3d(M.Grid3D(nx, ny, nz, 1.0), x, w, None, out_f32=True)
     ref = N.conv3d(_np(x).reshape(nz, ny, nx, cin), _np(w)).reshape(-1, cout)
     assert _rel(_np(y), ref) < 2e-5
+
+
+# output channels that are cut unevenly (64 + 48, 48 + 32, 48 + 48 + 16), with the bias, the ReLU, the mask and the
+# BF16 output of every launch
+@pytest.mark.parametrize("shape", [(3, 17, 9), (5, 33, 70), (1, 1, 1)])
+@pytest.mark.parametrize("cin,cout", [(16, 112), (32, 112), (48, 80), (48, 112), (64, 80), (64, 112)])
+def test_conv3d_uneven_channel_cuts_vs_oracle(mf3d, shape, cin, cout):
+    """FP32 output: 2e-5 of the largest value, as above.  BF16 output: rounded to 8 significant bits, so a value v
+    in [2^e, 2^(e+1)) is off by at most half of 2^(e-7), that is 2^-8 |v|, more."""
+    M = mf3d
+    r = np.random.default_rng(cin * 37 + cout + sum(shape))
+    nz, ny, nx = shape
+    x = _bf(r.normal(size=(nz * ny * nx, cin)))
+    w = _bf(r.normal(size=(cout, 27, cin)) / np.sqrt(27 * cin))
+    mask = _bf(r.normal(size=(nz * ny * nx, cout)))
+    import torch
+    bias = torch.from_numpy(r.normal(size=cout).astype(np.float32)).cuda()
+    g = M.Grid3D(nx, ny, nz, 1.0)
+    ref = N.conv3d(_np(x).reshape(nz, ny, nx, cin), _np(w)).reshape(-1, cout) + _np(bias)
+    assert _rel(_np(M.nn_conv3d(g, x, w, bias, out_f32=True)), ref) < 2e-5
+    y = _np(M.nn_conv3d(g, x, w, bias, relu=True, mask=mask))
+    assert _rel(y, np.maximum(ref, 0.0) * (_np(mask) > 0)) < 2e-5 + 2.0 ** -8
