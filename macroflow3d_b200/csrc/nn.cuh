@@ -701,7 +701,7 @@ int mf3d_nn_conv3d_wgrad(const mf3d_grid* g, int cin, int cout, const void* x, c
         if (cin < 16 || cout < 16) throw Error(MF3D_E_INVALID, "convolution channels must be multiples of 16 in [16, 128]");
         const nn::Dims d{g->nx, g->ny, g->nz};
         const size_t part = nn::WarmStartNet::wgrad_plan(d, cin, cout).part_floats;
-        DevMem scratch(part * sizeof(float));
+        StreamMem scratch(part * sizeof(float), (cudaStream_t)stream);
         int* err = ws_err_flag();
         nn::WarmStartNet::wgrad((cudaStream_t)stream, d, cin, cout, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy,
                                 dw, db, scratch.as<float>(), part, 0, err);
