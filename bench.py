@@ -397,8 +397,9 @@ def ensemble_shapes(seed, count):
 def ensemble_steps(M, prec, count, steps, warmup, seed, tune_reps=3):
     """Monte Carlo ensemble: `count` realisations of uneven grids (sigma^2 = 2, lambda = 6, seed
     + r), each step = set-up from K + PCG to ||r||/||b|| <= 1e-10 + face velocity for every
-    realisation.  Batched (mf3d_batch_*: one graph for all) against looping single solves
-    (one HeadSolver per distinct grid, reused as FlowWorkspace is)."""
+    realisation.  As one ensemble (mf3d_batch_*: the larger realisations by their own graphs on four
+    streams, more than four small ones as one batch; the record's "batched" figures) against looping single
+    solves (one HeadSolver per distinct grid, reused as FlowWorkspace is)."""
     import torch
     shapes = ensemble_shapes(seed, count)
     grids = [M.Grid3D(nx, ny, nz, 1.0) for nx, ny, nz in shapes]
@@ -449,7 +450,8 @@ def _ensemble_arms(M, b, solvers, grids, shapes, bc, cfg, Ks, hs, velocities, ti
     stream = torch.cuda.current_stream()
     b.set_K(Ks)
     tuning = b.autotune(tune_reps) if tune_reps > 0 else []
-    note(f"ensemble: autotuned {len(tuning)} positions; batched steps")
+    note(f"ensemble: {len(tuning)} positions of batched sweeps tuned"
+         + ("" if tuning else " (every realisation is solved side by side)") + "; steps as one ensemble")
 
     def bstep():
         b.set_K(Ks)
