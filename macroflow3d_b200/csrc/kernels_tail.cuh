@@ -201,8 +201,9 @@ __device__ __forceinline__ void tail2_body(const Tail2Args& a, const TI* __restr
 // From x = 0 the V-cycle on a level is a linear map of its b: dense_map_kernel runs the tail's own cycle
 // on every unit vector when K is set (one CTA per cell, its x is the column) and dense_apply_kernel applies
 // the matrix, a row per warp, instead of some hundred dependent half-sweeps.  The result is the cycle's up
-// to rounding, in FP64.  512 cells (2 MB): 2.8 us from L2, 5.5 from memory, the map 57 us a K; 960 cells 10 us; the
-// cluster kernel takes 25 us from 16^3 and 57 us from 24 x 20 x 16 cells, the one-CTA tail 150 us.
+// to rounding, in FP64.  512 cells (2 MB): 2.8 us from L2, 5.5 from memory, the map 57 us a K with 8^3 and 2^3
+// levels below; 960 cells 10 us; the cluster kernel takes 25 us from 16^3 and 57 us from 24 x 20 x 16 cells, the
+// one-CTA tail 150 us.
 // cells of the first level that is solved this way, at most: with levels below it, when it is the coarsest one
 // (of at least DN_SWEEPS sweeps), and where what would serve otherwise is slow
 constexpr int DN_MAX = 512, DN_MAX_LAST = 384, DN_SWEEPS = 20, DN_MAX_SLOW = 1024;

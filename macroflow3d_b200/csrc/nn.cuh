@@ -341,8 +341,8 @@ class WarmStartNet {
         float* out;
         __nv_bfloat16* dout;
         float* lpart;
-        // backward: gradient buffers (BF16 for the tensor-core operands, FP32 accumulators)
-        __nv_bfloat16 *g0, *g1; // [V0 x 128] ping-pong gradient buffers, sized for the widest level use
+        // backward: gradient buffers (BF16, the tensor core's operands)
+        __nv_bfloat16 *g0, *g1; // [V0 x 48] ping-pong, as large as the widest level's use (48 channels at L0)
         __nv_bfloat16 *sk0, *sk1, *sk2; // gradients of the skip connections at L0 (16), L1 (32), L2 (64)
         float* part;
         size_t part_floats;
