@@ -204,9 +204,8 @@ __device__ __forceinline__ void tail2_body(const Tail2Args& a, const TI* __restr
 // to rounding, in FP64.  512 cells (2 MB): 2.8 us from L2, 5.5 from memory, the map 57 us a K with 8^3 and 2^3
 // levels below; 960 cells 10 us; the cluster kernel takes 25 us from 16^3 and 57 us from 24 x 20 x 16 cells, the
 // one-CTA tail 150 us.
-// cells of the first level that is solved this way, at most: with levels below it, when it is the coarsest one
-// (of at least DN_SWEEPS sweeps), and where what would serve otherwise is slow
-constexpr int DN_MAX = 512, DN_MAX_LAST = 384, DN_SWEEPS = 20, DN_MAX_SLOW = 1024;
+constexpr int DN_MAX = 1024; // cells of the first level that is solved this way, at most
+constexpr int DN_SWEEPS_FEW = 20, DN_SWEEPS_MANY = 50; // coarsest sweeps: fewer do not pay, more pay on less
 constexpr int DN_NT = 128; // threads per unit vector: cheap barriers, and every vector of 8^3 cells resident at once
 __global__ void __launch_bounds__(DN_NT, 8) dense_map_kernel(const Tail2Args a, int ld, double* __restrict__ M) {
     const int col = blockIdx.x;

@@ -1100,23 +1100,23 @@ template <class T, class TC> class VCycle : public VCycleBase {
     // or the one-CTA tail serves.
     //
     // The matrix costs a cycle per cell when K is set and saves time in every V-cycle, so it has to pay within
-    // the solve's own cycles: 8 or 9 to 1e-10, 5 or 6 to 1e-6 (set_K, solve in ms; with the matrix | the cluster).
-    // D_ with levels below it, 50 coarsest sweeps: 512 cells (64^3) 0.15 + 0.92 | 0.13 + 1.00.  D_ the coarsest level:
-    // 216 cells 0.10 + 0.50 | 0.05 + 0.63, 343 cells 0.14 + 0.46 | 0.05 + 0.61, 512 cells 0.17 + 0.50 | 0.05 + 0.65 (paid
-    // after 4, 5 and 7 cycles), 1000 cells 0.44 + 0.68 | 0.05 + 0.94 (14 cycles), 1728 cells 1.11 + 0.42 | 0.04 + 0.90 (20
-    // cycles); 216 cells with 5 sweeps 0.06 + 0.59 | 0.05 + 0.58.  A grid that is one level needs 1 to 3 cycles when
-    // its sweeps are many: 343 cells, 400 sweeps 0.68 + 0.08 | 0.02 + 0.24.  The one-CTA tail, and the cluster where a
-    // coarsest level has more cells of a colour than threads, take 100 us a cycle instead of 30 to 60: a larger
-    // matrix pays there (9 x 11 x 10 cells 0.55 + 0.76 | 0.05 + 1.56).
+    // the solve's own cycles: 8 to 20 to 1e-10 (set_K + solve in ms; with the matrix | the cluster, 8 or 9 cycles).
+    // D_ with levels below it, 50 coarsest sweeps: 512 cells (64^3) 0.15 + 0.92 | 0.13 + 1.00, 1000 cells (20^3, with 125
+    // below) 0.18 + 0.42 | 0.05 + 0.62.  D_ the coarsest level: 216 cells 0.10 + 0.50 | 0.05 + 0.63, 512 cells 0.17 + 0.50 |
+    // 0.05 + 0.66 (paid after 7 cycles), 729 cells 0.32 + 0.65 | 0.05 + 0.97 (8), 1000 cells 0.44 + 0.68 | 0.05 + 0.94 (13, and
+    // 6 where the cluster has more cells of a colour than threads: 9 x 11 x 10 0.55 + 0.76 | 0.05 + 1.56), 1728 cells 1.11 +
+    // 0.42 | 0.04 + 0.91 (20).  With 400 sweeps a matrix of 1000 cells above 125 takes 0.72 + 0.42, one of the 125 0.36 +
+    // 0.51; with 5 sweeps one of 216 0.06 + 0.59, the cluster 0.05 + 0.58.  A grid that is one level needs 1 to 3 cycles when its
+    // sweeps are many: 343 cells, 400 sweeps 0.68 + 0.08 | 0.02 + 0.24.
     int dense_level(int nl) const { // D_, or -1
         const bool cluster = cp_.Lc >= 0;
         const int Ls = cluster ? cp_.Lc : Lt_;
         if (nl == 1 || std::getenv("MF3D_NO_CLUSTER_TAIL") || std::getenv("MF3D_NO_MATRIX")) return -1;
-        const bool kept = cluster && cp_.a.L[cp_.a.nlev - 1].hcap <= CT_NT; // its sweeps run from registers
+        // (a coarsest level of at most 64 cells is swept by one warp of each column's CTA: cheap whatever the count)
+        const bool many = cluster && coarse_ > DN_SWEEPS_MANY && G_[nl - 1].n > 64;
         int D = Ls;
-        while (D < nl - 1 && G_[D].n > (size_t)(cluster ? DN_MAX : DN_MAX_SLOW)) ++D;
-        if (D == nl - 1 && (G_[D].n > (size_t)(kept ? DN_MAX_LAST : DN_MAX_SLOW) || (cluster && coarse_ < DN_SWEEPS)))
-            return -1;
+        while (D < nl - 1 && G_[D].n > (size_t)(many ? DN_MAX / 2 : DN_MAX)) ++D;
+        if (D == nl - 1 && (G_[D].n > (size_t)DN_MAX || (cluster && coarse_ < DN_SWEEPS_FEW))) return -1;
         if (D < Lt_ || (D > Ls && !(pre_ == 2 && post_ == 2))) return -1;
         size_t smem = 0; // of the cycle that builds the matrix
         for (int l = D; l < nl; ++l) smem += 8 * ((size_t)(G_[l].nx + 2) * (G_[l].ny + 2) * (G_[l].nz + 2) + G_[l].n);

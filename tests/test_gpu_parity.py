@@ -699,13 +699,14 @@ def _coarse_way(s):
 
 
 # where the matrix of the coarsest levels pays within a solve's own cycles and where it does not: too many cells
-# (1728; 512 whose cluster sweeps run from registers), a grid that is one level, few sweeps; at the limits (343 cells;
-# 512 with levels below; 990 with more cells of a colour than the cluster has threads, and 990 with fewer)
+# (1728, 1100), a grid that is one level, few sweeps; at the limits (1000 coarsest cells; 1000 with levels below, and
+# with many sweeps 125 of them; 512 of a full hierarchy; 20 sweeps)
 @pytest.mark.parametrize("shape,levels,sweeps,way", [
-    ((24, 24, 24), 2, 50, "cluster"), ((8, 16, 16), 1, 400, "cluster"), ((7, 7, 7), 1, 50, "cluster"),
-    ((32, 32, 32), 3, 50, "cluster"), ((28, 28, 28), 3, 5, "cluster"), ((36, 44, 40), 3, 50, "cluster"),
-    ((28, 28, 28), 3, 50, "bricks_matrix"), ((28, 28, 28), 3, 20, "bricks_matrix"),
-    ((64, 64, 64), 16, 50, "bricks_matrix"), ((20, 20, 20), 3, 50, "bricks_matrix"),
+    ((24, 24, 24), 2, 50, "cluster"), ((44, 40, 40), 3, 50, "cluster"), ((8, 16, 16), 1, 400, "cluster"),
+    ((7, 7, 7), 1, 50, "cluster"), ((28, 28, 28), 3, 5, "cluster"),
+    ((20, 20, 20), 2, 50, "bricks_matrix"), ((40, 40, 40), 3, 50, "bricks_matrix"),
+    ((28, 28, 28), 3, 20, "bricks_matrix"), ((64, 64, 64), 16, 50, "bricks_matrix"), ((64, 64, 64), 16, 400, "bricks_matrix"),
+    ((20, 20, 20), 3, 50, "bricks_matrix"), ((20, 20, 20), 3, 400, "bricks_matrix"),
     ((40, 44, 36), 3, 50, "bricks_matrix")])
 def test_matrix_where_it_pays(mf3d, monkeypatch, shape, levels, sweeps, way):
     """The way chosen, its memory (a matrix of at most 1024 x 1024), and the V-cycle against the cluster's: the same
@@ -732,6 +733,8 @@ def test_matrix_where_it_pays(mf3d, monkeypatch, shape, levels, sweeps, way):
     assert size[0] - size[1] <= (10 << 20)
     if way == "cluster":
         assert size[0] == size[1]
+    if shape == (20, 20, 20) and levels == 3:  # a matrix of 1000 x 1000, or of 125 x 125
+        assert (size[0] - size[1] > (4 << 20)) == (sweeps == 50)
 
 
 # several batches of modes (the last one ragged), several parts along one axis or all (ragged, of one cell), no
